@@ -646,6 +646,7 @@ extern "C" int ctbb_backproject_device(const struct recon_metadata *mr, const fl
     Context &c = ctx();
     CTBB_TRY(require_device(c));
     std::lock_guard<std::mutex> lk(c.mu);
+    CTBB_TRY(staged_error_check());  // of a launch before
     return do_backproject(c, *mr, d_rebin, d_block);
 }
 
@@ -695,7 +696,7 @@ static int drained(Context &c, Body &&body)
                   cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
         return CTBB_ERR_CUDA;
     }
-    return st;
+    return st == CTBB_OK ? staged_error_check() : st;
 }
 
 static int reconstruct_device_in(Context &c, struct recon_metadata *mr, const float *d_scan, float *d_final,
@@ -1149,11 +1150,11 @@ static int prepared_block_params(Context &c, const struct recon_metadata &mb, co
 // the choice for the process.
 
 struct TuneKey {
-    int nx, ny, n_slices, nos, n_rows, nht, quad;
+    int nx, ny, n_slices, nos, n_rows, nht, quad, staged;  // staged: the staged form applies
     bool operator<(const TuneKey &o) const
     {
-        return std::tie(nx, ny, n_slices, nos, n_rows, nht, quad) <
-               std::tie(o.nx, o.ny, o.n_slices, o.nos, o.n_rows, o.nht, o.quad);
+        return std::tie(nx, ny, n_slices, nos, n_rows, nht, quad, staged) <
+               std::tie(o.nx, o.ny, o.n_slices, o.nos, o.n_rows, o.nht, o.quad, o.staged);
     }
 };
 
@@ -1180,7 +1181,10 @@ static int tune_reps()
 static int tuned_shape(Context &c, const BpParams &p_any, const BpShape &fallback, BpShape *out)
 {
     const bool quad = p_any.vscale != nullptr;
-    const TuneKey key{p_any.nx, p_any.ny, p_any.n_slices, p_any.nos, p_any.n_rows, p_any.nht, quad ? 1 : 0};
+    StagedShape st;
+    const bool staged = staged_shape(p_any, &st);
+    const TuneKey key{p_any.nx, p_any.ny, p_any.n_slices, p_any.nos, p_any.n_rows, p_any.nht, quad ? 1 : 0,
+                      staged ? 1 : 0};
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tuned.find(key);
@@ -1192,10 +1196,11 @@ static int tuned_shape(Context &c, const BpParams &p_any, const BpShape &fallbac
     std::vector<BpShape> cand = backproject_shape_candidates(quad);
     TuneEntry best;
     best.shape = fallback;
+    if (!staged) best.shape.staged = 0;
     double best_ms = 1e30;
     cudaEvent_t e0 = pooled_event(c), e1 = pooled_event(c);
     for (size_t k = 0; k < cand.size() && k < 8; ++k) {
-        if (cand[k].col && p_any.nht > kColumnMaxHalfTurns) continue;  // the window does not fit
+        if (cand[k].staged ? !staged : cand[k].col && p_any.nht > kColumnMaxHalfTurns) continue;  // does not fit
         BpParams p = p_any;
         p.col_zpt = cand[k].col ? cand[k].zpt : 0;
         p.warp_w = cand[k].warp_w;
@@ -1437,9 +1442,9 @@ extern "C" int ctbb_autotune_report(char *buf, size_t n)
         int len = snprintf(line, sizeof(line),
                            "%dx%dx%d nos %d rows %d nht %d %s: %s zpt %d threads %d ctas/sm %d cta_w %d;", k.nx, k.ny,
                            k.n_slices, k.nos, k.n_rows, k.nht, k.quad ? "fp16" : "fp32",
-                           e.shape.col ? "column" : "tile",
+                           e.shape.staged ? "staged" : e.shape.col ? "column" : "tile",
                            e.shape.zpt, e.shape.threads, e.shape.min_blocks, e.shape.cta_w);
-        if (e.shape.col) {
+        if (e.shape.col || e.shape.staged) {
             out.append(line, (size_t)std::max(0, std::min(len, (int)sizeof(line) - 1)));
             len = snprintf(line, sizeof(line), " angle chunks %d;", e.shape.achunks);
         }
@@ -1447,7 +1452,7 @@ extern "C" int ctbb_autotune_report(char *buf, size_t n)
         const std::vector<BpShape> &cc = k.quad ? cqq : cq;
         for (int i = 0; i < e.n && i < (int)cc.size(); ++i) {
             if (e.ms[i] <= 0.0) continue;  // not a candidate for this window
-            len = snprintf(line, sizeof(line), " %s%d/%d/%d/%dx%d/a%d %.3f ms", cc[i].col ? "c" : "t", cc[i].zpt,
+            len = snprintf(line, sizeof(line), " %s%d/%d/%d/%dx%d/a%d %.3f ms", cc[i].staged ? "s" : cc[i].col ? "c" : "t", cc[i].zpt,
                            cc[i].threads, cc[i].min_blocks, cc[i].cta_w, cc[i].warp_w, cc[i].achunks, e.ms[i]);
             out.append(line, (size_t)std::max(0, std::min(len, (int)sizeof(line) - 1)));
         }

@@ -19,8 +19,9 @@
 // interpolation) use FMA and reciprocals.  The reference's pi' = 3.1415368979f
 // is used where it uses it.
 //
-// GB300 mapping.  Two forms share the arithmetic below.  The column form (the
-// default, backproject_column_tile) gives a thread the (x, y) column over up to
+// GB300 mapping.  Three forms share the arithmetic below.  The staged form
+// (backproject_staged.cu) is the default wherever its conditions hold
+// (staged_shape).  The column form (backproject_column_tile) gives a thread the (x, y) column over up to
 // 32 slices: per angle it computes the geometry of each half turn once and
 // parks it in shared memory, then runs the slices in sub-chunks of 8, each
 // fetching all of a visit's footprints before it uses any (one wait on the
@@ -41,6 +42,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
@@ -49,6 +51,7 @@
 #include <vector>
 
 #include "backproject.h"
+#include "backproject_device.cuh"
 #include "ctbb_internal.h"
 #include "cuda_util.cuh"
 
@@ -56,72 +59,6 @@ namespace ctbb {
 
 namespace {
 
-
-constexpr float kQ = 0.6f;
-// slices per sub-chunk: the unit of the flat / inner / other decision
-constexpr int kSub = 8;
-
-// interp2 drops a sample when q_idx > R*nht - 2, which only the last half
-// turn can reach.  Its weight still counts, so the decision is a jump in the
-// image; near it the reference's own float q_idx decides.  This recomputes that
-// q_idx with the reference's operations and rounding (asin through double,
-// i.e. correctly rounded); it runs only when the fast coordinate is within
-// kBorderBand rows of the border.
-__device__ __forceinline__ bool last_turn_sample_valid(const BpParams &p, float x, float y, float theta,
-                                                    float s, float c, float phat, float z, int k)
-{
-    float asn = (float)asin((double)__fdiv_rn(phat, p.rf));
-    float ray = __fdiv_rn(__fmul_rn(p.z_rot, __fsub_rn(theta, asn)), p.two_pi);
-    float lhat = __fsub_rn(__fsub_rn(__fsqrt_rn(__fsub_rn(p.rf2, __fmul_rn(phat, phat))), __fmul_rn(x, c)),
-                           __fmul_rn(y, s));
-    float qhat = __fdiv_rn(__fsub_rn(z, ray), __fmul_rn(lhat, p.tan_cone));
-    float q_idx = __fadd_rn(__fmul_rn(__fdiv_rn(__fadd_rn(qhat, 1.0f), 2.0f), (float)p.n_rows - 1.0f),
-                            (float)(k * p.n_rows));
-    return !(q_idx > (float)(p.n_rows * p.nht - 2)) && !(q_idx < 0.0f);
-}
-
-constexpr float kBorderBand = 1e-3f;
-// inner chunks: |q| <= kInnerMax keeps every row below R-1 after rounding;
-// rows kRowMargin below the last-turn border are far from its band
-constexpr float kInnerMax = 0.999f;
-constexpr float kRowMargin = 0.01f;
-// half-turn window margin (angle rounding is ~1e-6 half turns)
-constexpr float kWindowMargin = 0.01f;
-
-// p_idx = p / (r_f fai / 2) + 2 cc as the reference rounds it (division, then
-// add), used where the interp2 border decision is close.
-__device__ __forceinline__ float p_index_exact(const BpParams &p, float phat)
-{
-    return __fadd_rn(__fdiv_rn(phat, p.ds_half), p.two_cc);
-}
-
-// asin(a) for |a| <= 0.5 as a + a^3 P(a^2), P of degree 4 fitted here by
-// weighted least squares on Chebyshev nodes (max error 0.67 ulp in float);
-// larger |a| (only the corners of very wide fields) fall back to asinf.
-__device__ __forceinline__ float asin_fast(float a)
-{
-    if (fabsf(a) > 0.5f) return asinf(a);
-    float t = a * a;
-    float p = fmaf(t, 0.042095037962576944f, 0.024220510033133892f);
-    p = fmaf(t, p, 0.04546249911296045f);
-    p = fmaf(t, p, 0.07495353339646753f);
-    p = fmaf(t, p, 0.16666751488866943f);
-    return fmaf(a * t, p, a);
-}
-
-// Row floors through the float unit: for |ql| < 2^22, ql + 1.5 2^23 rounded
-// down is exactly 1.5 2^23 + floor(ql) (the binade [2^23, 2^24) has unit
-// spacing), so one packed add gives both the floor as a float (t - 1.5 2^23,
-// exact) and as an integer (the bits of t are kFloorMagicBits + floor(ql)).
-// The row address is then view + bits(t) * row stride with the view's base
-// moved back by kFloorMagicBits rows (64-bit modular arithmetic, folded into
-// BpParams::rebin_rows on the host): one multiply-add, no conversion.
-constexpr float kFloorMagic = 12582912.0f;       // 1.5 * 2^23
-constexpr uint32_t kFloorMagicBits = 0x4B400000u;  // its bits
-__device__ __forceinline__ float2 row_floor(float2 ql)
-{
-    return __fadd2_rd(ql, make_float2(kFloorMagic, kFloorMagic));
-}
 
 // The 2x2 footprint {(p, row), (p+1, row), (p, row+1), (p+1, row+1)} of a
 // view, row in [0, R-2] given as t = kFloorMagic + row (row_floor);
@@ -150,12 +87,6 @@ __device__ __forceinline__ void fetch_footprint(uint64_t view_rows, int nos, flo
         v11 = __ldg(r0 + nos + 1);
     }
 }
-
-// Packed FP32 pairs (sm_100 family): one instruction for two lanes.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
 // NOS > 0: the row length as a compile-time constant (the second row of a
 // footprint is then an immediate offset); 0: taken from p.nos.
@@ -459,7 +390,6 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) backproject_kernel(BpPara
 }
 
 // ---- column form --------------------------------------------------------
-enum { kOutScaled = 0, kOutPartial = 1, kOutFirst = 2, kOutMiddle = 3, kOutLast = 4 };
 
 // A thread owns the voxel column (x, y) over up to ZMAX slices (zpt of them,
 // in sub-chunks of SUB = 8).  Per angle, the geometry of every half turn in
@@ -1002,6 +932,12 @@ int make_backproject_params(const struct recon_metadata &mr, const BackprojectTa
     p.n_rows = (int)cg.n_rows;
     p.nht = t.nht;
     p.n_half = t.n_half;
+    p.n_views = 0;
+    for (size_t v = 0; v < t.views.size(); v += 4) {
+        uint32_t row;
+        std::memcpy(&row, &t.views[v], sizeof(row));
+        p.n_views = std::max(p.n_views, (int)row + 1);
+    }
     p.pix_x = rp.recon_fov / (float)rp.nx;
     p.pix_y = rp.recon_fov / (float)rp.ny;
     p.x_c = (float)(rp.nx - 1) / 2.0f;
@@ -1104,6 +1040,18 @@ bool bp_column_form()
     return v;
 }
 
+// Whether a knob names the column or the slice-chunk form or a shape of theirs.
+bool bp_shape_named()
+{
+    static bool v = [] {
+        for (const char *k : {"CTBB_BP_FORM", "CTBB_BP_COL_ZPT", "CTBB_BP_MINB", "CTBB_BP_CTA_W", "CTBB_BP_WARP_W",
+                              "CTBB_BP_ZPT", "CTBB_BP_THREADS"})
+            if (getenv(k)) return true;
+        return false;
+    }();
+    return v;
+}
+
 // Slices per thread of the column form (32; 16 or 8).
 int bp_column_zpt()
 {
@@ -1121,6 +1069,7 @@ BpShape fit_bp_shape(const BpShape &s, int nht)
     BpShape t;  // the slice-chunk form's default
     t.cta_w = s.cta_w;
     t.warp_w = s.warp_w;
+    t.staged = s.staged;
     return t;
 }
 
@@ -1162,6 +1111,8 @@ BpShape default_bp_shape(int zpt, bool quad)
         const char *a = getenv("CTBB_BP_ACHUNKS");
         const int ach = a ? atoi(a) : 16;
         s.achunks = (ach >= 1 && ach <= kMaxAngleChunks) ? ach : 16;
+        // the staged form, unless a knob names another one's shape
+        if (!bp_shape_named()) s.staged = s.achunks;
         return s;
     }
     if (quad) return BpShape{};
@@ -1197,10 +1148,32 @@ int with_column_shape(const BpShape &s, F &&f)
     return CTBB_ERR_ARGUMENT;
 }
 
+namespace {
+
+// Angle chunks a launch of this shape splits a block's angles into.
+int shape_chunks(const BpParams &p, const BpShape &shape)
+{
+    StagedShape st;
+    if (shape.staged && staged_shape(p, &st)) return staged_chunks(p, st, shape.staged);
+    return shape.col ? shape.achunks : 1;
+}
+
+int launch_combine(const BpParams &p, cudaStream_t stream)
+{
+    const size_t n = (size_t)p.n_slices * p.nx * p.ny;
+    const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 152 * 16);
+    backproject_combine_kernel<<<blocks, 256, 0, stream>>>(p.partial, p.out, n, p.n_achunks, p.out_scale);
+    count_launch();
+    CTBB_CUDA_TRY(cudaGetLastError());
+    return CTBB_OK;
+}
+
+}  // namespace
+
 size_t backproject_partial_bytes(const BpParams &p, const BpShape &shape)
 {
-    if (!shape.col || shape.achunks <= 1) return 0;
-    return (size_t)shape.achunks * p.n_slices * p.nx * p.ny * sizeof(float);
+    const int chunks = shape_chunks(p, shape);
+    return chunks <= 1 ? 0 : (size_t)chunks * p.n_slices * p.nx * p.ny * sizeof(float);
 }
 
 int launch_backproject_params(const BpParams &p_in, const BpShape &shape, cudaStream_t stream, void *scratch,
@@ -1209,10 +1182,16 @@ int launch_backproject_params(const BpParams &p_in, const BpShape &shape, cudaSt
     BpParams p = p_in;
     p.n_achunks = 1;
     p.partial = nullptr;
+    const int chunks = shape_chunks(p, shape);
     const size_t part_bytes = backproject_partial_bytes(p, shape);
-    if (part_bytes && scratch && scratch_bytes >= part_bytes && shape.achunks <= p.n_half) {
-        p.n_achunks = shape.achunks;
+    if (part_bytes && scratch && scratch_bytes >= part_bytes && chunks <= p.n_half) {
+        p.n_achunks = chunks;
         p.partial = static_cast<float *>(scratch);
+    }
+    StagedShape st;
+    if (shape.staged && staged_shape(p, &st)) {
+        CTBB_TRY(launch_backproject_staged(p, st, stream));
+        return p.partial ? launch_combine(p, stream) : CTBB_OK;
     }
     const bool quad = p.vscale != nullptr;
     const dim3 grid = grid_of(p, shape);
@@ -1242,13 +1221,7 @@ int launch_backproject_params(const BpParams &p_in, const BpShape &shape, cudaSt
         }));
         count_launch();
         CTBB_CUDA_TRY(cudaGetLastError());
-        if (p.partial) {
-            const size_t n = (size_t)p.n_slices * p.nx * p.ny;
-            const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 152 * 16);
-            backproject_combine_kernel<<<blocks, 256, 0, stream>>>(p.partial, p.out, n, p.n_achunks, p.out_scale);
-            count_launch();
-            CTBB_CUDA_TRY(cudaGetLastError());
-        }
+        if (p.partial) CTBB_TRY(launch_combine(p, stream));
         return CTBB_OK;
     }
     CTBB_TRY(with_shape(shape, quad, false, [&](auto z, auto mb, auto t, auto q) -> int {
@@ -1275,12 +1248,74 @@ int launch_backproject(const struct recon_metadata &mr, const BackprojectTables 
     return launch_backproject_params(p, s, stream, scratch, scratch_bytes);
 }
 
-size_t backproject_batch_bytes(size_t n_blocks) { return n_blocks * sizeof(BpParams) + (n_blocks + 1) * 4 + 256; }
+// the blocks' TMA descriptors first (aligned by the allocation), then their
+// parameters, then the tile starts
+size_t backproject_batch_bytes(size_t n_blocks)
+{
+    return n_blocks * (staged_map_bytes() + sizeof(BpParams)) + (n_blocks + 1) * 4 + 256;
+}
+
+namespace {
+
+// The blocks of a batch that take the staged form: those of one staged shape
+// together, one launch per angle chunk.
+int launch_staged_batch(const std::vector<BpParams> &blocks, int chunks, void *d_buf, size_t buf_bytes,
+                        cudaStream_t stream)
+{
+    std::vector<StagedShape> shapes(blocks.size());
+    std::vector<StagedShape> kinds;
+    for (size_t b = 0; b < blocks.size(); ++b) {
+        if (!staged_shape(blocks[b], &shapes[b])) {
+            set_error("backproject batch: a block does not fit the staged form");
+            return CTBB_ERR_ARGUMENT;
+        }
+        if (std::find(kinds.begin(), kinds.end(), shapes[b]) == kinds.end()) kinds.push_back(shapes[b]);
+    }
+    if (backproject_batch_bytes(blocks.size()) > buf_bytes) {
+        set_error("backproject batch: parameter buffer too small");
+        return CTBB_ERR_ARGUMENT;
+    }
+    for (const StagedShape &kind : kinds) {
+        std::vector<BpParams> group;
+        std::vector<unsigned> start(1, 0);
+        std::vector<unsigned char> maps;
+        int n_ac = std::max(1, chunks);
+        for (size_t b = 0; b < blocks.size(); ++b) {
+            if (!(shapes[b] == kind)) continue;
+            group.push_back(blocks[b]);
+            alignas(64) unsigned char map[256];
+            CTBB_TRY(staged_map(blocks[b], kind, map));
+            maps.insert(maps.end(), map, map + staged_map_bytes());
+            n_ac = std::min(n_ac, blocks[b].n_half);
+            const unsigned long long next = (unsigned long long)start.back() + staged_tiles(blocks[b], kind);
+            if (next >= (1ull << 31)) {
+                set_error("backproject batch: more than 2^31 CTA tiles");
+                return CTBB_ERR_ARGUMENT;
+            }
+            start.push_back((unsigned)next);
+        }
+        char *d_maps = static_cast<char *>(d_buf);
+        BpParams *d_params = reinterpret_cast<BpParams *>(d_maps + maps.size());
+        unsigned *d_start = reinterpret_cast<unsigned *>(d_params + group.size());
+        CTBB_CUDA_TRY(cudaMemcpyAsync(d_maps, maps.data(), maps.size(), cudaMemcpyHostToDevice, stream));
+        CTBB_CUDA_TRY(cudaMemcpyAsync(d_params, group.data(), group.size() * sizeof(BpParams), cudaMemcpyHostToDevice,
+                                      stream));
+        CTBB_CUDA_TRY(cudaMemcpyAsync(d_start, start.data(), start.size() * sizeof(unsigned), cudaMemcpyHostToDevice,
+                                      stream));
+        for (int ac = 0; ac < n_ac; ++ac)
+            CTBB_TRY(launch_backproject_staged_batch(d_params, d_start, d_maps, start.back(), (int)group.size(), ac,
+                                                     n_ac, kind, stream));
+    }
+    return CTBB_OK;
+}
+
+}  // namespace
 
 int launch_backproject_batch(const std::vector<BpParams> &blocks, const BpShape &shape, void *d_buf, size_t buf_bytes,
                              cudaStream_t stream)
 {
     if (blocks.empty()) return CTBB_OK;
+    if (shape.staged) return launch_staged_batch(blocks, shape.staged, d_buf, buf_bytes, stream);
     const bool quad = blocks[0].vscale != nullptr;
     for (const BpParams &p : blocks)
         if ((p.vscale != nullptr) != quad || p.nos != blocks[0].nos) {
@@ -1367,6 +1402,7 @@ std::vector<BpShape> backproject_shape_candidates(bool quad)
 {
     // 128-thread CTAs are 32 x 4 (cta_w 32) or 16 x 8 (cta_w 16) voxel columns
     std::vector<BpShape> c;
+    c.push_back(BpShape{32, 128, 8, 16, 8, 1, 16, 16});
     c.push_back(BpShape{32, 128, 8, 16, 8, 1, 16});
     c.push_back(BpShape{32, 128, 7, 16, 8, 1, 16});
     c.push_back(BpShape{32, 128, 8, 32, 8, 1, 16});

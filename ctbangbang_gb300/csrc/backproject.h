@@ -34,6 +34,7 @@ struct BpParams {
     const float *theta;    // [n_half][nht] theta (the last-turn border recheck)
     const float *zpos;     // [n_slices_block]
     int nx, ny, n_slices, nos, n_rows, nht, n_half;
+    int n_views;           // views the rows buffer holds (one past the last of the table's row indices)
     float pix_x, pix_y, x_c, y_c, x0, y0;  // x = pix_x * (xi - x_c) + x0
     float ds_half;         // r_f fai / 2
     float inv_ds_half;     // 1 / ds_half
@@ -66,14 +67,49 @@ struct BpParams {
 // achunks (column form): the half-turn angles split into that many chunks,
 // each run by CTAs of its own that write unscaled partial image sums, which a
 // second kernel adds in chunk order (smaller CTA lifetimes: a shorter tail).
+// staged: the angle chunks of the staged form (backproject_staged.cu), which
+// takes a block in place of the shape's own form wherever staged_shape allows
+// it (at most: staged_chunks); 0: not staged.
 struct BpShape {
-    int zpt = 8, threads = 128, min_blocks = 7, cta_w = 64, warp_w = 8, col = 0, achunks = 1;
+    int zpt = 8, threads = 128, min_blocks = 7, cta_w = 64, warp_w = 8, col = 0, achunks = 1, staged = 0;
     bool operator==(const BpShape &o) const
     {
         return zpt == o.zpt && threads == o.threads && min_blocks == o.min_blocks && cta_w == o.cta_w &&
-               warp_w == o.warp_w && col == o.col && achunks == o.achunks;
+               warp_w == o.warp_w && col == o.col && achunks == o.achunks && staged == o.staged;
     }
 };
+// The staged form's tile for a block: column warps of a CTA (16 x 8 voxel
+// columns with 4, 8 x 8 with 2), elements of a staged detector row, bytes of
+// half of the box buffer.
+struct StagedShape {
+    int cw = 4, pitch = 56;
+    unsigned half_bytes = 0;
+    bool operator==(const StagedShape &o) const
+    {
+        return cw == o.cw && pitch == o.pitch && half_bytes == o.half_bytes;
+    }
+};
+// The staged form's tile for a block's parameters; false where the form does
+// not apply (FP16 footprint words, rows off 16-byte boundaries, pixels whose footprint is too wide,
+// more than 32 slices, voxels near the source's circle).
+bool staged_shape(const BpParams &p, StagedShape *out);
+int launch_backproject_staged(const BpParams &p, const StagedShape &s, cudaStream_t stream);
+// Angle chunk ac of n_ac of n blocks of one staged shape, total CTA tiles.
+// d_maps: the blocks' TMA descriptors (staged_map, staged_map_bytes() each, 64-byte aligned).
+int launch_backproject_staged_batch(const BpParams *d_params, const unsigned *d_start, const void *d_maps,
+                                    unsigned total, int n, int ac, int n_ac, const StagedShape &s,
+                                    cudaStream_t stream);
+size_t staged_map_bytes();
+int staged_map(const BpParams &p, const StagedShape &s, void *out);
+unsigned staged_tiles(const BpParams &p, const StagedShape &s);
+// Angle chunks of a block, at most limit: half of it where the tiles of one
+// chunk fill the GPU already (two CTAs per SM), since each CTA lists its
+// visits anew (16 chunks against 8: 3.91 -> 3.85 ms at 256^2, 12.78 -> 12.68 ms
+// at 512^2, but 0.22 -> 0.24 ms for a scan of 48^2).
+int staged_chunks(const BpParams &p, const StagedShape &s, int limit);
+// CTBB_ERR_CUDA once a staged kernel's bounded wait has run out (read after a
+// stream synchronisation, or at the next call).
+int staged_error_check();
 constexpr int kColumnMaxHalfTurns = 8;
 constexpr int kMaxAngleChunks = 16;  // the most angle chunks a launch shape uses
 // The shape the environment knobs (CTBB_BP_*) name: the column form (unless
