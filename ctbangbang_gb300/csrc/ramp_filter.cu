@@ -10,8 +10,10 @@
 // GB300 design: FP32 FFT convolution in shared memory.  Two real rows are
 // packed into one complex row (x_a + i x_b); because the kernel is real the
 // real and imaginary parts of the inverse transform are the two filtered rows.
-// CTAs are persistent and loop over row pairs.  For M = 4096 (row lengths
-// 1025..2048, every built-in scanner) ramp_fft4096_kernel runs 16 x 16 x 16
+// CTAs are persistent and loop over row pairs.  Row lengths 1025..1536 (every
+// built-in scanner) take ramp_fft3072_kernel (16 x 16 x 12), see there; any M
+// of at least 2 N - 1 gives the same convolution.  For M = 4096 (row lengths
+// 1537..2048) ramp_fft4096_kernel runs 16 x 16 x 16
 // radix-16 passes: thread j owns butterfly j of every pass, the first forward
 // pass reads the rows from HBM (inputs >= M/2 are the zero padding), the last
 // forward pass, the spectrum multiply and the first inverse pass stay in
@@ -79,6 +81,7 @@ struct FftParams {
     int m;               // transform size (power of two)
     int log2m;
     const float2 *spectrum;  // H[k] / M, [m]
+    int diff;            // the 3072-point kernel transforms x[i] - x[i - 1], i <= n
 };
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b)
@@ -417,6 +420,186 @@ __global__ void __launch_bounds__(kFftThreads, MIN_BLOCKS)
     }
 }
 
+// ---- 3072-point transforms (16 x 16 x 12): row lengths 1025..1536.  A linear
+// convolution of N samples with 2 N - 1 taps needs M >= 2 N - 1 points, so 3072
+// serve these rows with three quarters of the 4096-point kernel's work.  The
+// same structure: inputs at M / 2 and beyond are the zero padding (first pass,
+// r >= 8) and are not needed after the last inverse pass; thread j of the two
+// middle passes (radix 12, j < 256) holds X[j + 256 r], which is what the
+// spectrum multiply and the first inverse pass take; the four radix-16 passes
+// are 192 butterflies (six of the eight warps).
+//
+// Difference form (plan->diff).  A ramp kernel takes the large low frequencies
+// of a row to a small output, so the rounding of the forward transform, which
+// scales with the whole row, ends up at 1e-5 of the output.  The same
+// convolution is sum_k F[l - k] (x[k] - x[k - 1]) with F the running sum of
+// the taps and x zero outside its row (N + 1 differences, N <= 1535): the
+// differences of a row are some thirty times smaller than the row, and so is
+// the rounding (against 64 bits on 40 001 rows of 1344: 1.0e-5 of the result's
+// norm plain, 1.4e-7 as differences, for 4 % of the time).  Taken when F's white-noise gain is no larger than the taps'.
+//
+// Bound by the L1 data pipe
+// (70 %: shared-memory round trips and the twiddle tables) and the barriers
+// between passes, which four CTAs per SM (64 registers) overlap better than
+// three or two (40 001 rows of 1344: 270, 276 and 320 us; the 4096-point
+// kernel 313 us, at 9.3e-6).
+constexpr int kM3072 = 3072;
+// float2 slots of a buffer: rows of 12 padded to 13 (the widest layout used)
+constexpr int kBuf3072 = 13 * 256;
+
+// In-place 3-point DFT of (a, b, c), outputs in natural order.
+template <int SIGN>
+__device__ __forceinline__ void dft3(float2 &a, float2 &b, float2 &c)
+{
+    constexpr float h = SIGN < 0 ? -0.86602540378443865f : 0.86602540378443865f;
+    const float2 s = cadd(b, c), d = csub(b, c);
+    const float2 t = __ffma2_rn(s, make_float2(-0.5f, -0.5f), a);
+    a = cadd(a, s);
+    // t +- i h d
+    b = __ffma2_rn(make_float2(-d.y, d.x), make_float2(h, h), t);
+    c = __ffma2_rn(make_float2(d.y, -d.x), make_float2(h, h), t);
+}
+
+// z * exp(SIGN 2 pi i e / 12), e = 1, 2, 4
+template <int SIGN, int E>
+__device__ __forceinline__ float2 w12(float2 z)
+{
+    constexpr float r = 0.86602540378443865f;
+    constexpr float c = E == 1 ? r : (E == 2 ? 0.5f : -0.5f);
+    constexpr float sn = (SIGN < 0 ? -1.0f : 1.0f) * (E == 1 ? 0.5f : r);
+    return make_float2(fmaf(z.x, c, -z.y * sn), fmaf(z.x, sn, z.y * c));
+}
+
+// 12-point DFT in registers, V[k] = sum_n v[n] exp(SIGN 2 pi i n k / 12), as
+// 3 x 4: n = 4 a + b, k = c + 3 d.
+template <int SIGN>
+__device__ __forceinline__ void dft12(float2 (&v)[12])
+{
+#pragma unroll
+    for (int b = 0; b < 4; ++b) dft3<SIGN>(v[b], v[4 + b], v[8 + b]);
+    // element (b, c) sits at 4 c + b: times exp(SIGN 2 pi i b c / 12)
+    v[4 + 1] = w12<SIGN, 1>(v[4 + 1]);
+    v[4 + 2] = w12<SIGN, 2>(v[4 + 2]);
+    v[4 + 3] = mul_omega4<SIGN>(v[4 + 3]);
+    v[8 + 1] = w12<SIGN, 2>(v[8 + 1]);
+    v[8 + 2] = w12<SIGN, 4>(v[8 + 2]);
+    v[8 + 3] = make_float2(-v[8 + 3].x, -v[8 + 3].y);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) dft4<SIGN>(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+    // element (c, d) now sits at 4 c + d; output k = c + 3 d
+    float2 t[12];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int d = 0; d < 4; ++d) t[c + 3 * d] = v[4 * c + d];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) v[k] = t[k];
+}
+
+__global__ void __launch_bounds__(kFftThreads, 4)
+    ramp_fft3072_kernel(FftParams p, const float2 *__restrict__ tw)
+{
+    extern __shared__ float2 smem[];
+    float2 *buf_a = smem;
+    float2 *buf_b = smem + kBuf3072;
+    const float2 *tw_f2 = tw, *tw_f3 = tw + 15 * 16, *tw_i2 = tw_f3 + 11 * 256, *tw_i3 = tw_i2 + 15 * 12;
+    const int j = threadIdx.x;
+    const bool outer = j < 192;  // butterflies of the radix-16 passes
+    // padded offsets as base + compile-time stride (one slot per 16, see pad)
+    const int rd = j + (j >> 4);                         // j + 192 r at 204 r, j + 256 r at 272 r
+    const int out2 = ((j >> 4) << 8) + (j & 15);
+    const int wr2 = out2 + (out2 >> 4);
+    // the first inverse pass writes rows of 12 (slots of 13), the second reads
+    // j + 192 r from them and writes blocks of 192 (slots of 204)
+    const int q12 = j / 12, m12 = j - 12 * q12;
+    const size_t n_pairs = (p.n_lines + 1) / 2;
+    for (size_t pair = blockIdx.x; pair < n_pairs; pair += gridDim.x) {
+        const size_t la = 2 * pair, lb = la + 1;
+        const bool has_b = lb < p.n_lines;
+        float *ra = p.lines + la * (size_t)p.n;
+        float *rb = p.lines + lb * (size_t)p.n;
+        float2 v[16];
+        if (outer) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int idx = j + 192 * r;
+                float xa = 0.0f, xb = 0.0f;
+                if (idx < p.n) {
+                    xa = __ldg(ra + idx);
+                    if (has_b) xb = __ldg(rb + idx);
+                }
+                v[r] = make_float2(xa, xb);
+            }
+            if (p.diff) {
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const int idx = j + 192 * r;
+                    const bool in = idx > 0 && idx <= p.n;
+                    v[8 + r] = make_float2(in ? __ldg(ra + idx - 1) : 0.0f, in && has_b ? __ldg(rb + idx - 1) : 0.0f);
+                }
+#pragma unroll
+                for (int r = 0; r < 8; ++r) v[r] = csub(v[r], v[8 + r]);
+            }
+#pragma unroll
+            for (int r = 8; r < 16; ++r) v[r] = make_float2(0.0f, 0.0f);
+            dft16<-1, true>(v);
+#pragma unroll
+            for (int r = 0; r < 16; ++r) buf_a[17 * j + r] = v[r];
+        }
+        __syncthreads();
+        if (outer) {
+#pragma unroll
+            for (int r = 0; r < 16; ++r) v[r] = buf_a[rd + 204 * r];
+            apply_twiddles<-1, 16>(v, tw_f2, j & 15);
+            dft16<-1, false>(v);
+#pragma unroll
+            for (int r = 0; r < 16; ++r) buf_b[wr2 + 17 * r] = v[r];
+        }
+        __syncthreads();
+        {
+            float2 u[12];
+#pragma unroll
+            for (int r = 0; r < 12; ++r) u[r] = buf_b[rd + 272 * r];
+#pragma unroll
+            for (int r = 1; r < 12; ++r) u[r] = twiddle<-1>(u[r], __ldg(tw_f3 + (r - 1) * 256 + j));
+            dft12<-1>(u);
+            // kernel spectrum H / M, then the first inverse pass, in registers
+#pragma unroll
+            for (int r = 0; r < 12; ++r) u[r] = cmul(u[r], __ldg(p.spectrum + j + 256 * r));
+            dft12<1>(u);
+#pragma unroll
+            for (int r = 0; r < 12; ++r) buf_a[13 * j + r] = u[r];
+        }
+        __syncthreads();
+        if (outer) {
+#pragma unroll
+            for (int r = 0; r < 16; ++r) v[r] = buf_a[j + q12 + 208 * r];
+            apply_twiddles<1, 12>(v, tw_i2, m12);
+            dft16<1, false>(v);
+#pragma unroll
+            for (int r = 0; r < 16; ++r) buf_b[q12 * 204 + m12 + 12 * r] = v[r];
+        }
+        __syncthreads();
+        if (outer) {
+#pragma unroll
+            for (int r = 0; r < 16; ++r) v[r] = buf_b[j + 204 * r];
+            apply_twiddles<1, 192>(v, tw_i3, j);
+            dft16<1, false>(v);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int idx = j + 192 * r;
+                if (idx < p.n) {
+                    ra[idx] = v[r].x;
+                    if (has_b) rb[idx] = v[r].y;
+                }
+            }
+        }
+        // buf_a is rewritten next by the next pair's first pass: its last reads
+        // precede the barrier before this pass; buf_b is rewritten after the
+        // barrier that follows that first pass.
+    }
+}
+
 __global__ void __launch_bounds__(kFftThreads, 3) ramp_fft_kernel(FftParams p, const float2 *__restrict__ tw)
 {
     // twiddles come from the read-only cache (one table for every CTA), which
@@ -468,6 +651,7 @@ int fft4096_mode()
 
 int ramp_transform_size(int n)
 {
+    if (n > 1024 && n < kM3072 / 2) return kM3072;  // N + 1 differences, at most M / 2
     int m = 1;
     while (m < n) m <<= 1;
     return 2 * m;
@@ -493,18 +677,76 @@ int prepare_ramp_filter(const float *h_taps, int n, RampFilterPlan *plan, cudaSt
     int centre = (int)std::floor((2.0f * n - 1.0f) / 2.0f) + 1;
     for (int i = 0; i < n; ++i) F[2 * (size_t)i] = h_taps[centre + i];
     for (int i = m - n + 1; i < m; ++i) F[2 * (size_t)i] = h_taps[i - (m - n + 1) + 1];
-    ctbb_fft_radix2_double(F.data(), m, -1);
+    plan->diff = 0;
+    if (m == kM3072) {
+        // running sum of the taps over the lags -N + 1 .. N - 1, also taken at lag
+        // -N (the difference at k = N); zero there and below
+        std::vector<double> S(2 * (size_t)m, 0.0);
+        double sum = 0.0, e_taps = 0.0, e_sum = 0.0;
+        for (int lag = -n + 1; lag < n; ++lag) {
+            const size_t at = (size_t)(lag < 0 ? m + lag : lag);
+            sum += F[2 * at];
+            S[2 * at] = sum;
+            e_taps += F[2 * at] * F[2 * at];
+            e_sum += sum * sum;
+        }
+        if (e_sum <= e_taps) {
+            plan->diff = 1;
+            F.swap(S);
+        }
+    }
+    const double two_pi = 6.283185307179586476925286766559;
+    if (m == kM3072) {
+        // three interleaved 1024-point transforms, X[k] = sum_s w^(s k) E_s[k mod 1024]
+        const int third = m / 3;
+        std::vector<double> E(2 * (size_t)m);
+        for (int s = 0; s < 3; ++s) {
+            for (int i = 0; i < third; ++i)
+                for (int c = 0; c < 2; ++c) E[2 * (size_t)(s * third + i) + c] = F[2 * (size_t)(3 * i + s) + c];
+            ctbb_fft_radix2_double(&E[2 * (size_t)(s * third)], third, -1);
+        }
+        for (int k = 0; k < m; ++k) {
+            double re = 0.0, im = 0.0;
+            for (int s = 0; s < 3; ++s) {
+                const double a = -two_pi * (double)((long long)s * k % m) / (double)m;
+                const double wr = std::cos(a), wi = std::sin(a);
+                const double *e = &E[2 * (size_t)(s * third + k % third)];
+                re += e[0] * wr - e[1] * wi;
+                im += e[0] * wi + e[1] * wr;
+            }
+            F[2 * (size_t)k] = re;
+            F[2 * (size_t)k + 1] = im;
+        }
+    } else {
+        ctbb_fft_radix2_double(F.data(), m, -1);
+    }
     std::vector<float2> H(m), tw(m);
     for (int k = 0; k < m; ++k) H[k] = make_float2((float)(F[2 * (size_t)k] / m), (float)(F[2 * (size_t)k + 1] / m));
-    const double two_pi = 6.283185307179586476925286766559;
     for (int t = 0; t < m; ++t) {
         double a = -two_pi * (double)t / (double)m;
         tw[t] = make_float2((float)std::cos(a), (float)std::sin(a));
     }
-    // radix-16 tables of the 4096-point kernel, [r - 1][k]: pass 2
-    // exp(-2 pi i r k / 256) (k < 16), pass 3 exp(-2 pi i r k / 4096) (k < 256)
+    // pass tables of the 4096-point kernel, [r - 1][k]: pass 2
+    // exp(-2 pi i r k / 256) (k < 16), pass 3 exp(-2 pi i r k / 4096) (k < 256);
+    // of the 3072-point kernel: forward exp(-2 pi i r k / 256) (k < 16) and
+    // exp(-2 pi i r k / 3072) (r < 12, k < 256), inverse exp(-2 pi i r k / 192)
+    // (k < 12) and exp(-2 pi i r k / 3072) (k < 192), conjugated when applied
     std::vector<float2> tw16(kTw16Entries);
-    for (int r = 1; r < 16; ++r) {
+    if (m == kM3072) {
+        tw16.clear();
+        auto table = [&](int radix, int nk, int of) {
+            for (int r = 1; r < radix; ++r)
+                for (int k = 0; k < nk; ++k) {
+                    const double a = -two_pi * (double)(r * k) / (double)of;
+                    tw16.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
+                }
+        };
+        table(16, 16, 256);
+        table(12, 256, m);
+        table(16, 12, 192);
+        table(16, 192, m);
+    }
+    for (int r = 1; m != kM3072 && r < 16; ++r) {
         for (int k = 0; k < 16; ++k) {
             double a = -two_pi * (double)(r * k) / 256.0;
             tw16[(r - 1) * 16 + k] = make_float2((float)std::cos(a), (float)std::sin(a));
@@ -514,7 +756,7 @@ int prepare_ramp_filter(const float *h_taps, int n, RampFilterPlan *plan, cudaSt
             tw16[15 * 16 + (r - 1) * 256 + k] = make_float2((float)std::cos(a), (float)std::sin(a));
         }
     }
-    size_t need = 2 * (size_t)m + kTw16Entries;
+    size_t need = 2 * (size_t)m + tw16.size();
     if (!plan->d_spectrum || plan->capacity < need) {
         if (plan->d_spectrum) cudaFree(plan->d_spectrum);
         plan->d_spectrum = nullptr;
@@ -525,7 +767,7 @@ int prepare_ramp_filter(const float *h_taps, int n, RampFilterPlan *plan, cudaSt
     plan->d_tw16 = plan->d_twiddle + m;
     CTBB_CUDA_TRY(cudaMemcpyAsync(plan->d_spectrum, H.data(), sizeof(float2) * m, cudaMemcpyHostToDevice, stream));
     CTBB_CUDA_TRY(cudaMemcpyAsync(plan->d_twiddle, tw.data(), sizeof(float2) * m, cudaMemcpyHostToDevice, stream));
-    CTBB_CUDA_TRY(cudaMemcpyAsync(plan->d_tw16, tw16.data(), sizeof(float2) * kTw16Entries,
+    CTBB_CUDA_TRY(cudaMemcpyAsync(plan->d_tw16, tw16.data(), sizeof(float2) * tw16.size(),
                                   cudaMemcpyHostToDevice, stream));
     // the host vectors die at return: make the copies complete first
     CTBB_CUDA_TRY(cudaStreamSynchronize(stream));
@@ -543,6 +785,7 @@ int launch_ramp_filter(const RampFilterPlan &plan, float *d_lines, size_t n_line
     p.log2m = 0;
     while ((1 << p.log2m) < p.m) p.log2m++;
     p.spectrum = plan.d_spectrum;
+    p.diff = plan.diff;
     auto padded = [](size_t m) { return m + ((m - 1) >> 4) + 1; };
     size_t smem = sizeof(float2) * 2 * padded((size_t)p.m);
     // the shared-memory limits are a per-device setting of each kernel
@@ -558,6 +801,8 @@ int launch_ramp_filter(const RampFilterPlan &plan, float *d_lines, size_t n_line
                                            (int)(sizeof(float2) * 2 * padded(kM4096))));
         CTBB_CUDA_TRY(cudaFuncSetAttribute(ramp_fft4096_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)(sizeof(float2) * 2 * padded(kM4096))));
+        CTBB_CUDA_TRY(cudaFuncSetAttribute(ramp_fft3072_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(sizeof(float2) * 2 * kBuf3072)));
         attr_devices.fetch_or(bit);
     }
     int per_sm = (int)std::max<size_t>(1, (size_t)(220 * 1024) / smem);
@@ -565,7 +810,10 @@ int launch_ramp_filter(const RampFilterPlan &plan, float *d_lines, size_t n_line
     size_t n_pairs = (n_lines + 1) / 2;
     int grid = (int)std::min<size_t>(n_pairs, (size_t)num_sms() * per_sm);
     int mode = fft4096_mode();
-    if (p.m == kM4096 && mode == 3) {
+    if (p.m == kM3072) {
+        grid = (int)std::min<size_t>(n_pairs, (size_t)num_sms() * 4);
+        ramp_fft3072_kernel<<<grid, kFftThreads, sizeof(float2) * 2 * kBuf3072, stream>>>(p, plan.d_tw16);
+    } else if (p.m == kM4096 && mode == 3) {
         ramp_fft4096_kernel<3><<<grid, kFftThreads, smem, stream>>>(p, plan.d_tw16, plan.d_tw16 + 15 * 16);
     } else if (p.m == kM4096 && mode == 2) {
         grid = (int)std::min<size_t>(n_pairs, (size_t)num_sms() * std::min(per_sm, 2));

@@ -14,10 +14,11 @@ constexpr int kMaxRampTransform = 8192;  // rows up to 4096 samples
 struct RampFilterPlan {
     int n = 0;                     // row length (n_channels_oversampled)
     int m = 0;                     // transform size
+    int diff = 0;                  // the spectrum is of the taps' running sum, for the rows' differences
     std::vector<float> taps;       // 2n host taps the spectrum was made from
     float2 *d_spectrum = nullptr;  // H/M [m], followed by the twiddle table [m]
     float2 *d_twiddle = nullptr;  // exp(-2 pi i t / m) [m]
-    float2 *d_tw16 = nullptr;     // radix-16 pass tables of the 4096-point kernel
+    float2 *d_tw16 = nullptr;     // pass tables of the 4096- or 3072-point kernel
     size_t capacity = 0;
 };
 
