@@ -87,20 +87,86 @@ __global__ void af_sup_kernel(AfParams p)
 
 __global__ void af_smooth_kernel(AfParams p)
 {
-    int proj = p.f0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (proj >= p.f1) return;
-    float w = __fdiv_rn(1.0f, (float)p.n_avg);
+    // the CTA's windows, weighted, in shared memory; the sum keeps the
+    // reference's order
+    extern __shared__ float win[];
+    const int first = p.f0 + blockIdx.x * blockDim.x, n = min((int)blockDim.x, p.f1 - first);
+    const float w = __fdiv_rn(1.0f, (float)p.n_avg);
+    const int max_idx = p.P - 1;
+    for (int i = threadIdx.x; i < n + p.n_avg - 1; i += blockDim.x)
+        win[i] = __fmul_rn(w, p.sup[min(max(first - p.avg_offset + i, 0), max_idx)]);
+    __syncthreads();
+    if ((int)threadIdx.x >= n) return;
     float acc = 0.0f;
-    int max_idx = p.P - 1;
-    for (int i = 0; i < p.n_avg; i++) {
-        int idx = proj - p.avg_offset + i;
-        idx = idx < 0 ? 0 : (idx > max_idx ? max_idx : idx);
-        acc = __fadd_rn(acc, __fmul_rn(w, p.sup[idx]));
-    }
-    p.smooth[proj] = acc;
+#pragma unroll 8
+    for (int i = 0; i < p.n_avg; i++) acc = __fadd_rn(acc, win[threadIdx.x + i]);
+    p.smooth[first + threadIdx.x] = acc;
 }
 
-__global__ void af_ecc_kernel(AfParams p)
+// eccentricity from the window's extremes (include/preprocessing.cuh:133-150)
+__device__ __forceinline__ void write_ecc(const AfParams &p, int proj, float vmax, float vmin)
+{
+    p.pmax[proj] = vmax;
+    p.pmin[proj] = vmin;
+    float e = __fsub_rn(1.0f, __fdiv_rn(vmin, vmax));
+    e = __fdiv_rn(__fsub_rn(e, 0.3f), __fsub_rn(0.5f, 0.3f));
+    float out;
+    if (e > 1) out = 1.0f;
+    else if (e < 0) out = 0.0f;
+    else out = e;
+    p.ecc[proj] = out;
+}
+
+// Extremes of every frame's window by doubling: after the pass of length len,
+// hi[i] is the maximum of len consecutive means from i (lo the minimum), and a
+// window is the union of two such runs.  Extremes do not depend on the order,
+// so this equals the reference's scan of the window (max from 0, min from
+// 10000, frames outside the scan repeated at its ends).  Instead of 2305
+// reads per frame (config 2), 12 passes over the CTA's 2560 means: 62 -> 9 us
+// for 11 264 frames.
+constexpr int kEccFrames = 256;
+constexpr size_t kEccSmem = 48 * 1024;
+
+__host__ __device__ constexpr size_t ecc_smem(int n_range)
+{
+    return 4 * sizeof(float) * (size_t)(kEccFrames + n_range - 1);
+}
+
+__global__ void __launch_bounds__(kEccFrames) af_ecc_kernel(AfParams p)
+{
+    extern __shared__ float win[];
+    const int first = p.f0 + blockIdx.x * kEccFrames, n = min(kEccFrames, p.f1 - first);
+    const int w = n + p.n_range - 1, stride = kEccFrames + p.n_range - 1;
+    float *hi = win, *lo = win + stride, *hi2 = win + 2 * stride, *lo2 = win + 3 * stride;
+    for (int i = threadIdx.x; i < w; i += kEccFrames) {
+        const int idx = first - p.range_offset + i;
+        const bool in = idx >= 0 && idx < p.P;  // a window past an end holds the end frame itself
+        const float v = in ? p.smooth[idx] : 0.0f;
+        hi[i] = fmaxf(v, 0.0f);
+        lo[i] = in ? fminf(v, 10000.0f) : 10000.0f;
+    }
+    __syncthreads();
+    int len = 1;
+    for (; 2 * len <= p.n_range; len *= 2) {
+        for (int i = threadIdx.x; i + 2 * len <= w; i += kEccFrames) {
+            hi2[i] = fmaxf(hi[i], hi[i + len]);
+            lo2[i] = fminf(lo[i], lo[i + len]);
+        }
+        __syncthreads();
+        float *t = hi;
+        hi = hi2;
+        hi2 = t;
+        t = lo;
+        lo = lo2;
+        lo2 = t;
+    }
+    const int i = threadIdx.x, j = i + p.n_range - len;
+    if (i < n) write_ecc(p, first + i, fmaxf(hi[i], hi[j]), fminf(lo[i], lo[j]));
+}
+
+// The same with one thread reading its whole window, for windows past the
+// shared memory of the kernel above (turns of more than 5600 frames).
+__global__ void af_ecc_long_kernel(AfParams p)
 {
     int proj = p.f0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (proj >= p.f1) return;
@@ -113,57 +179,101 @@ __global__ void af_ecc_kernel(AfParams p)
         if (v > vmax) vmax = v;
         if (v < vmin) vmin = v;
     }
-    p.pmax[proj] = vmax;
-    p.pmin[proj] = vmin;
-    float e = __fsub_rn(1.0f, __fdiv_rn(vmin, vmax));
-    e = __fdiv_rn(__fsub_rn(e, 0.3f), __fsub_rn(0.5f, 0.3f));
-    float out;
-    if (e > 1) out = 1.0f;
-    else if (e < 0) out = 0.0f;
-    else out = e;
-    p.ecc[proj] = out;
+    write_ecc(p, proj, vmax, vmin);
 }
 
-// rhs() of include/preprocessing.cuh:32-62, the window count split over a warp.
-__device__ float window_fraction(const AfParams &p, int start_idx, float T, int lane)
-{
-    int numel = p.n_range;
-    int max_idx = p.P - 1;
-    int diff = start_idx + (numel - 1);
-    if (diff < (numel - 1)) {
-        numel += start_idx;
-        start_idx = 0;
-    }
-    if (diff > max_idx) numel -= (diff - max_idx);
-    int count = 0;
-    for (int i = lane; i < numel; i += 32) count += (p.smooth[start_idx + i] > T) ? 1 : 0;
-    for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
-    const float inv_pi = 1.0f / kPiAf;
-    return __fmul_rn(__fmul_rn(inv_pi, (float)count), __fdiv_rn(1.0f, (float)p.n_proj_ffs));
-}
+// One warp per frame: the bisection of find_thresholds with the window count
+// of rhs() (include/preprocessing.cuh:32-62), an exact integer, split over the
+// lanes.  NV > 0: a lane keeps its NV values of the window in registers, so
+// that a step of the bisection reads nothing (a value beyond the window is
+// -inf, never above a threshold); NV = 0: windows of more than 2560 frames
+// are read again each step.  A value at or below the lower bound is never
+// counted again and one above the upper bound always is: once at most 256
+// values lie between, only those are kept and compared, 8 to a lane (after
+// three or four of the up to 21 steps on a window of 2305).  11 264 frames of
+// 2305: 101 us read again each step, 89 us all from registers, 70 us so.
+constexpr int kFew = 8;  // values per lane once few are left
 
-__global__ void af_threshold_kernel(AfParams p)
+template <int NV>
+__global__ void __launch_bounds__(256) af_threshold_kernel(AfParams p)
 {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    int proj = p.f0 + warp;
+    __shared__ float few[8][32 * kFew];
+    const int lane = threadIdx.x & 31;
+    const int proj = p.f0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (proj >= p.f1) return;
-    float lower = p.pmin[proj];
-    float upper = p.pmax[proj];
-    float T = __fdiv_rn(__fadd_rn(p.pmax[proj], p.pmin[proj]), 2.0f);
-    float lhs = __fmul_rn(__fmul_rn(kFMax, p.strength), p.ecc[proj]);
-    int start = proj - p.range_offset;
-    float rhs = window_fraction(p, start, T, lane);
+    // the window, cut at the scan's ends
+    const int begin = max(proj - p.range_offset, 0);
+    const int numel = min(proj - p.range_offset + p.n_range, p.P) - begin;
+    const float *win = p.smooth + begin;
+    float v[NV > 0 ? NV : 1];
+    if constexpr (NV > 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) v[k] = lane + 32 * k < numel ? win[lane + 32 * k] : -INFINITY;
+    }
+    int above = 0;  // values no longer kept that are above every further threshold
+    bool is_few = false;
+    auto count = [&](float T) {
+        int n = 0;
+        if (is_few || (NV > 0 && NV <= kFew)) {
+#pragma unroll
+            for (int k = 0; k < (NV > 0 ? min(NV, kFew) : 1); ++k) n += v[k] > T ? 1 : 0;
+        } else if constexpr (NV > 0) {
+            int m = 0;
+#pragma unroll
+            for (int k = 0; k < NV; k += 2) {
+                n += v[k] > T ? 1 : 0;
+                m += v[k + 1] > T ? 1 : 0;
+            }
+            n += m;
+        } else {
+            for (int i = lane; i < numel; i += 32) n += win[i] > T ? 1 : 0;
+        }
+        return __reduce_add_sync(0xffffffffu, n) + above;
+    };
+    const float inv_pi = 1.0f / kPiAf, inv_turn = __fdiv_rn(1.0f, (float)p.n_proj_ffs);
+    auto fraction = [&](int n) { return __fmul_rn(__fmul_rn(inv_pi, (float)n), inv_turn); };
+    float lower = p.pmin[proj], upper = p.pmax[proj];
+    int n_lower = numel, n_upper = 0;  // values above each bound (at most, for the first)
+    float T = __fdiv_rn(__fadd_rn(upper, lower), 2.0f);
+    const float lhs = __fmul_rn(__fmul_rn(kFMax, p.strength), p.ecc[proj]);
+    int n = count(T);
+    float rhs = fraction(n);
     int iter = 0;
-    // (|lhs - rhs| / lhs) > 0.01 with the float quotient promoted to double
-    while ((double)__fdiv_rn(fabsf(__fsub_rn(lhs, rhs)), lhs) > 0.01) {
+    // the reference compares the float quotient, promoted to double, with
+    // 0.01; no float lies between 0.01f and 0.01
+    while (__fdiv_rn(fabsf(__fsub_rn(lhs, rhs)), lhs) > 0.01f) {
         if (iter >= 20) break;
         iter += 1;
-        if (rhs > lhs) lower = T;
-        else if (rhs < lhs) upper = T;
-        else break;
+        if (rhs > lhs) {
+            lower = T;
+            n_lower = n;
+        } else if (rhs < lhs) {
+            upper = T;
+            n_upper = n;
+        } else {
+            break;
+        }
+        if constexpr (NV > kFew) {
+            if (!is_few && n_lower - n_upper <= 32 * kFew) {
+                float *kept = few[threadIdx.x >> 5];
+                int at = 0;
+#pragma unroll
+                for (int k = 0; k < NV; ++k) {
+                    const bool keep = v[k] > lower && v[k] <= upper;
+                    const unsigned who = __ballot_sync(0xffffffffu, keep);
+                    if (keep) kept[at + __popc(who & ((1u << lane) - 1u))] = v[k];
+                    at += __popc(who);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < kFew; ++k) v[k] = lane + 32 * k < at ? kept[lane + 32 * k] : -INFINITY;
+                above = n_upper;
+                is_few = true;
+            }
+        }
         T = __fdiv_rn(__fadd_rn(lower, upper), 2.0f);
-        rhs = window_fraction(p, start, T, lane);
+        n = count(T);
+        rhs = fraction(n);
     }
     if (lane == 0) p.thr[proj] = T;
 }
@@ -237,17 +347,26 @@ __device__ __noinline__ float smooth_sample(const AfParams &p, int gp, int gr, i
 #pragma unroll 1
     for (int ii = 0; ii < 5; ii++) {
         int c = gc + ii - 2;
-#pragma unroll 1
-        for (int jj = 0; jj < 5; jj++) {
-            int r = gr + jj - 2;
+        if (c < 0 || c >= p.N) continue;
+        // the channel's 25 taps are all fetched before the first is added (a
+        // list is often shorter than a warp, its latency the whole cost)
+        float x[5][5];
+#pragma unroll
+        for (int jj = 0; jj < 5; jj++)
 #pragma unroll
             for (int kk = 0; kk < 5; kk++) {
-                int f = gp + kk - 2;
-                if (c < 0 || c >= p.N || r < 0 || r >= p.R || f < 0 || f >= p.P) continue;
-                float x = __ldg(p.raw + (size_t)f * frame + (size_t)r * p.N + c);
-                val = __fadd_rn(val, __fmul_rn(x, (float)(tri1(ii) + tri1(jj) + tri1(kk) + 1)));
+                const int r = gr + jj - 2, f = gp + kk - 2;
+                const bool in = r >= 0 && r < p.R && f >= 0 && f < p.P;
+                x[jj][kk] = in ? __ldg(p.raw + (size_t)f * frame + (size_t)r * p.N + c) : 0.0f;
             }
-        }
+#pragma unroll
+        for (int jj = 0; jj < 5; jj++)
+#pragma unroll
+            for (int kk = 0; kk < 5; kk++) {
+                const int r = gr + jj - 2, f = gp + kk - 2;
+                if (r < 0 || r >= p.R || f < 0 || f >= p.P) continue;
+                val = __fadd_rn(val, __fmul_rn(x[jj][kk], (float)(tri1(ii) + tri1(jj) + tri1(kk) + 1)));
+            }
     }
     return __fmul_rn(__fdiv_rn(1.0f, norm), val);
 }
@@ -261,11 +380,13 @@ __device__ __noinline__ float smooth_sample(const AfParams &p, int gp, int gr, i
 // result as the tiled form.
 constexpr int kSmoothListMax = 1024;
 
-__global__ void __launch_bounds__(256) af_filter_stream_kernel(AfParams p)
+__global__ void __launch_bounds__(256, 4) af_filter_stream_kernel(AfParams p)
 {
     __shared__ int list[kSmoothListMax];
     __shared__ int n_list;
-    int gp = p.f0 + blockIdx.x;
+    // last frame first: the end of the range is what the maxima's pass left in
+    // L2, and its beginning is what the rebinning reads first
+    int gp = p.f1 - 1 - (int)blockIdx.x;
     size_t frame = (size_t)p.R * p.N;
     const float4 *src = reinterpret_cast<const float4 *>(p.raw + (size_t)gp * frame);
     float4 *dst = reinterpret_cast<float4 *>(p.out + (size_t)gp * frame);
@@ -398,15 +519,23 @@ int af_launch(AfParams p, int sup0, int sup1, int smooth0, int smooth1, int out0
     if (smooth1 > smooth0) {
         p.f0 = smooth0;
         p.f1 = smooth1;
-        af_smooth_kernel<<<(smooth1 - smooth0 + 127) / 128, 128, 0, stream>>>(p);
+        af_smooth_kernel<<<(smooth1 - smooth0 + 127) / 128, 128, (size_t)(127 + p.n_avg) * sizeof(float), stream>>>(p);
         ++launches;
     }
     if (out1 > out0 && thresholds) {
         int n = out1 - out0;
         p.f0 = out0;
         p.f1 = out1;
-        af_ecc_kernel<<<(n + 127) / 128, 128, 0, stream>>>(p);
-        af_threshold_kernel<<<(n * 32 + 255) / 256, 256, 0, stream>>>(p);
+        if (ecc_smem(p.n_range) <= kEccSmem)
+            af_ecc_kernel<<<(n + kEccFrames - 1) / kEccFrames, kEccFrames, ecc_smem(p.n_range), stream>>>(p);
+        else
+            af_ecc_long_kernel<<<(n + 127) / 128, 128, 0, stream>>>(p);
+        const int ctas = (n + 7) / 8;
+        if (p.n_range <= 8 * 32) af_threshold_kernel<8><<<ctas, 256, 0, stream>>>(p);
+        else if (p.n_range <= 20 * 32) af_threshold_kernel<20><<<ctas, 256, 0, stream>>>(p);
+        else if (p.n_range <= 40 * 32) af_threshold_kernel<40><<<ctas, 256, 0, stream>>>(p);
+        else if (p.n_range <= 80 * 32) af_threshold_kernel<80><<<ctas, 256, 0, stream>>>(p);
+        else af_threshold_kernel<0><<<ctas, 256, 0, stream>>>(p);
         launches += 2;
     }
     if (out1 > out0 && output) {
