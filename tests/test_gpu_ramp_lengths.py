@@ -1,5 +1,6 @@
-"""The FFT ramp filter at the row lengths where its transform changes (1024 /
-1025, 1536 / 1537) and inside each range, with one row, an odd and an even
+"""The FFT ramp filter at the row lengths where its transform changes (powers of
+two, 1024 / 1025, 1535 / 1536) and inside each range (short transforms share a
+CTA), with one row, an odd and an even
 number of rows, against the oracle's double-precision FFT convolution; bar as
 in the other filter tests, 2e-5 of the largest sample."""
 import ctypes as C
@@ -14,7 +15,7 @@ pytestmark = pytest.mark.gpu
 fptr = lambda a: a.ctypes.data_as(C.POINTER(C.c_float))
 
 
-@pytest.mark.parametrize("n_os", [1024, 1026, 1344, 1535, 1536, 1537])
+@pytest.mark.parametrize("n_os", [5, 16, 48, 128, 129, 256, 500, 1024, 1026, 1344, 1535, 1536, 1537])
 @pytest.mark.parametrize("n_lines", [1, 2, 777])
 def test_ramp_filter_vs_oracle(oracle_lib, lib, n_os, n_lines):
     torch = pytest.importorskip("torch")
