@@ -66,10 +66,24 @@ float r_fr_f(float da, float dr, const struct ct_geom &cg)
     return std::sqrt((cg.r_f + dr) * (cg.r_f + dr) + da * da);
 }
 
-float get_beta_idx_f(float beta, const float *lookup, int n)
+// get_beta_idx with the search begun where the last one ended: every entry
+// before it is below the last beta, so for a beta no smaller the first entry
+// that is not below it is the same as from 0 (1472 searches of 1472 entries
+// took the host 1.1 ms of every rebin call).
+struct BetaSearch {
+    const float *lookup;
+    int n, from = 0;
+    float last = -INFINITY;
+};
+
+float get_beta_idx_f(float beta, BetaSearch &b)
 {
-    int lo = 0;
+    const float *lookup = b.lookup;
+    const int n = b.n;
+    int lo = beta >= b.last ? b.from : 0;
     while (beta > lookup[lo] && lo < (n - 1)) lo++;
+    b.from = lo;
+    b.last = beta;
     if (lo == 0) lo++;
     return (float)lo - 1.0f + (beta - lookup[lo - 1]) / (lookup[lo] - lookup[lo - 1]);
 }
@@ -145,6 +159,7 @@ int build_rebin_tables(const struct recon_metadata &mr, RebinTables *t)
             lk2[i] = beta_rk_f((float)da, (float)dr, (float)i, 0, cg);
         }
         t->focal.assign(2 * (size_t)Nos, FocalTerm{});
+        BetaSearch at1{lk1.data(), N}, at2{lk2.data(), N};
         float dal1 = d_alpha_r_f((float)da, (float)-dr, cg) * (float)cg.n_proj_ffs / (2.0f * pi);
         float dal2 = d_alpha_r_f((float)da, (float)dr, cg) * (float)cg.n_proj_ffs / (2.0f * pi);
         t->focal_offset[0] = dal1;
@@ -154,8 +169,8 @@ int build_rebin_tables(const struct recon_metadata &mr, RebinTables *t)
                                  cg.r_f / r_fr_f(0.0f, (float)-dr, cg));
             float b2 = std::asin(((float)c - 2.0f * cg.central_channel) * (cg.fan_angle_increment / 2.0f) *
                                  cg.r_f / r_fr_f(0.0f, (float)dr, cg));
-            set_tap(0, c, get_beta_idx_f(b1, lk1.data(), N), N);
-            set_tap(1, c, get_beta_idx_f(b2, lk2.data(), N), N);
+            set_tap(0, c, get_beta_idx_f(b1, at1), N);
+            set_tap(1, c, get_beta_idx_f(b2, at2), N);
             t->focal[c].t_alpha = b1 * (float)cg.n_proj_ffs / (2.0f * pi);
             t->focal[(size_t)Nos + c].t_alpha = b2 * (float)cg.n_proj_ffs / (2.0f * pi);
         }
@@ -177,9 +192,10 @@ int build_rebin_tables(const struct recon_metadata &mr, RebinTables *t)
             t->focal[0 * (size_t)N + ch].t_alpha = b1 * (float)cg.n_proj_ffs / (2.0f * pi);
             t->focal[1 * (size_t)N + ch].t_alpha = b2 * (float)cg.n_proj_ffs / (2.0f * pi);
         }
+        BetaSearch at{lookup.data(), Nos};
         for (int c = 0; c < Nos; ++c) {
             float beta = std::asin((c - 2 * cg.central_channel) * (cg.fan_angle_increment / 2));
-            set_tap(0, c, get_beta_idx_f(beta, lookup.data(), Nos), Nos);
+            set_tap(0, c, get_beta_idx_f(beta, at), Nos);
         }
     } else if (t->n_ffs == 4) {
         // rebin_affs_cpu :424-601
@@ -202,13 +218,14 @@ int build_rebin_tables(const struct recon_metadata &mr, RebinTables *t)
                 else lk2[2 * ch + (q - 2)] = b;
             }
         }
+        BetaSearch at1{lk1.data(), Nos}, at2{lk2.data(), Nos};
         for (int c = 0; c < Nos; ++c) {
             float b1 = std::asin((c - 2 * cg.central_channel) * (cg.fan_angle_increment / 2) * cg.r_f /
                                  r_fr_f(0.0f, (float)-dr, cg));
             float b2 = std::asin((c - 2 * cg.central_channel) * (cg.fan_angle_increment / 2) * cg.r_f /
                                  r_fr_f(0.0f, (float)dr, cg));
-            set_tap(0, c, get_beta_idx_f(b1, lk1.data(), Nos), Nos);
-            set_tap(1, c, get_beta_idx_f(b2, lk2.data(), Nos), Nos);
+            set_tap(0, c, get_beta_idx_f(b1, at1), Nos);
+            set_tap(1, c, get_beta_idx_f(b2, at2), Nos);
         }
     } else {
         set_error("rebin: unsupported n_ffs %d", t->n_ffs);
