@@ -18,7 +18,7 @@ LIB = os.path.join(HERE, "libctbb_gb300.so")
 
 CUDA_SOURCES = [
     "abi.cu", "adaptive_filter.cu", "rebin.cu", "ramp_filter.cu", "ramp_tc.cu",
-    "backproject.cu", "backproject_staged.cu", "finalize.cu",
+    "backproject.cu", "backproject_staged.cu", "finalize.cu", "tma.cu",
 ]
 HOST_SOURCES = ["planner.cpp", "dicom.cpp", "server.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

@@ -30,6 +30,7 @@
 #include "ramp_filter.h"
 #include "ramp_tc.h"
 #include "rebin.h"
+#include "tma.cuh"
 
 namespace ctbb {
 
@@ -569,6 +570,7 @@ extern "C" int ctbb_rebin_device(const struct recon_metadata *mr, const float *d
     Context &c = ctx();
     CTBB_TRY(require_device(c));
     std::lock_guard<std::mutex> lk(c.mu);
+    CTBB_TRY(copy_error_check());  // of a launch before
     return do_rebin(c, *mr, d_raw, d_rebin);
 }
 
@@ -646,7 +648,7 @@ extern "C" int ctbb_backproject_device(const struct recon_metadata *mr, const fl
     Context &c = ctx();
     CTBB_TRY(require_device(c));
     std::lock_guard<std::mutex> lk(c.mu);
-    CTBB_TRY(staged_error_check());  // of a launch before
+    CTBB_TRY(copy_error_check());  // of a launch before
     return do_backproject(c, *mr, d_rebin, d_block);
 }
 
@@ -696,7 +698,7 @@ static int drained(Context &c, Body &&body)
                   cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
         return CTBB_ERR_CUDA;
     }
-    return st == CTBB_OK ? staged_error_check() : st;
+    return st == CTBB_OK ? copy_error_check() : st;
 }
 
 static int reconstruct_device_in(Context &c, struct recon_metadata *mr, const float *d_scan, float *d_final,
@@ -1527,7 +1529,7 @@ extern "C" int ctbb_rebin_filter(struct recon_metadata *mr)
     if (mr->flags.testing && mr->ctd.rebin)
         CTBB_CUDA_TRY(cudaMemcpyAsync(mr->ctd.rebin, d_rebin, rebin_bytes, cudaMemcpyDeviceToHost, c.stream));
     CTBB_CUDA_TRY(cudaStreamSynchronize(c.stream));
-    return CTBB_OK;
+    return copy_error_check();
 }
 
 extern "C" int ctbb_backproject(struct recon_metadata *mr)
@@ -1556,7 +1558,7 @@ extern "C" int ctbb_backproject(struct recon_metadata *mr)
     CTBB_CUDA_TRY(cudaFree(mr->ctd.d_rebin));
     if (c.our_d_rebin == mr->ctd.d_rebin) c.our_d_rebin = nullptr;
     mr->ctd.d_rebin = nullptr;
-    return CTBB_OK;
+    return copy_error_check();
 }
 
 static int finalize_common(struct recon_metadata *mr, float mu_water)

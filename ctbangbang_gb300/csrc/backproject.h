@@ -107,9 +107,6 @@ unsigned staged_tiles(const BpParams &p, const StagedShape &s);
 // visits anew (16 chunks against 8: 3.91 -> 3.85 ms at 256^2, 12.78 -> 12.68 ms
 // at 512^2, but 0.22 -> 0.24 ms for a scan of 48^2).
 int staged_chunks(const BpParams &p, const StagedShape &s, int limit);
-// CTBB_ERR_CUDA once a staged kernel's bounded wait has run out (read after a
-// stream synchronisation, or at the next call).
-int staged_error_check();
 constexpr int kColumnMaxHalfTurns = 8;
 constexpr int kMaxAngleChunks = 16;  // the most angle chunks a launch shape uses
 // The shape the environment knobs (CTBB_BP_*) name: the column form (unless

@@ -28,17 +28,16 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
-#include <mutex>
 #include <vector>
 
 #include "backproject.h"
 #include "backproject_device.cuh"
 #include "ctbb_internal.h"
 #include "cuda_util.cuh"
+#include "tma.cuh"
 
 namespace ctbb {
 
@@ -49,7 +48,6 @@ constexpr int kRecords = 192;       // visits of one segment of angles
 constexpr int kTileY = 8;           // voxel columns of a tile along y
 constexpr int kBoxRows = 8;         // detector rows of a TMA copy
 constexpr float kBoxMargin = 0.05f; // rows / channels added around the box's bounds
-constexpr uint32_t kWaitTries = 100000, kSuspendNs = 20000;
 // class of a visit for a slice group
 enum : uint32_t { kSkip = 0, kFlat = 1, kInner = 2, kOther = 3, kBorder = 4, kOff = 5 };
 
@@ -77,39 +75,6 @@ __host__ __device__ inline StagedLayout staged_layout(int cw, unsigned half_byte
     l.counts = l.bars + 4u * 8u;
     l.total = l.counts + 32u * 4u;
     return l;
-}
-
-__device__ __forceinline__ uint32_t smem_address(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void barrier_init(uint32_t bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void barrier_arrive_expect(uint32_t bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-// Waits for the phase of the given parity, in at most kWaitTries tries that
-// may each sleep kSuspendNs (about two seconds); false when they ran out.
-__device__ __forceinline__ bool barrier_wait(uint32_t bar, uint32_t parity)
-{
-    uint32_t left;
-    asm volatile(
-        "{\n .reg .pred p, q;\n"
-        " mov.u32 %0, %3;\n"
-        "WAIT_%=:\n"
-        " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %4;\n"
-        " @p bra DONE_%=;\n"
-        " sub.u32 %0, %0, 1;\n"
-        " setp.ne.u32 q, %0, 0;\n"
-        " @q bra WAIT_%=;\n"
-        "DONE_%=:\n}\n"
-        : "=&r"(left)
-        : "r"(bar), "r"(parity), "n"(kWaitTries), "n"(kSuspendNs)
-        : "memory");
-    return left != 0;
 }
 
 // kBoxRows rows of PITCH samples of the rows buffer seen as one matrix
@@ -544,15 +509,9 @@ __device__ __forceinline__ void backproject_staged_tile(const Params &p, int bx,
         if (!alive) break;
     }
     if (!alive) {
-        // a wait ran out: report it, give copies in flight time to land in
-        // this CTA's shared memory, and leave
+        // a wait ran out: report it and leave
         *reinterpret_cast<volatile int *>(error) = 1;
-        uint64_t t0, t1;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-        for (int n = 0; n < (1 << 20); ++n) {
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-            if (t1 - t0 > 2000000ull) break;
-        }
+        wait_for_stray_copies();
         return;
     }
     if (!inside) return;
@@ -630,52 +589,14 @@ int with_staged(const StagedShape &s, F &&f)
     return CTBB_ERR_ARGUMENT;
 }
 
-// The word a kernel sets when a bounded wait runs out, in pinned host memory
-// so that it is read without a copy.
-int *error_word()
-{
-    static std::once_flag once;
-    static int *word = nullptr;
-    std::call_once(once, [] {
-        void *v = nullptr;
-        if (cudaHostAlloc(&v, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
-            word = static_cast<int *>(v);
-            *word = 0;
-        }
-    });
-    return word;
-}
-
-using EncodeTiled = decltype(&cuTensorMapEncodeTiled);
-
 // The rows buffer of a block as a matrix of view rows, box kBoxRows x pitch
 // samples; samples past its edges read as zeros.
 int rows_map(const BpParams &p, int pitch, CUtensorMap *map)
 {
-    static EncodeTiled encode = [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            f = nullptr;
-        return reinterpret_cast<EncodeTiled>(f);
-    }();
-    if (!encode) {
-        set_error("backproject: cuTensorMapEncodeTiled not available");
-        return CTBB_ERR_CUDA;
-    }
     const cuuint64_t dims[2] = {(cuuint64_t)p.nos, (cuuint64_t)p.n_views * (cuuint64_t)p.n_rows};
     const cuuint64_t strides[1] = {dims[0] * 4};
     const cuuint32_t box[2] = {(cuuint32_t)pitch, (cuuint32_t)kBoxRows};
-    const cuuint32_t step[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(p.rebin), dims, strides, box,
-                              step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        set_error("backproject: cuTensorMapEncodeTiled failed (%d)", (int)r);
-        return CTBB_ERR_CUDA;
-    }
-    return CTBB_OK;
+    return tensor_map_f32(map, p.rebin, 2, dims, strides, box);
 }
 
 int raise_smem_limit(const void *kernel)
@@ -728,11 +649,8 @@ bool staged_shape(const BpParams &p, StagedShape *out)
 
 int launch_backproject_staged(const BpParams &p, const StagedShape &s, cudaStream_t stream)
 {
-    int *err = error_word();
-    if (!err) {
-        set_error("backproject: no pinned memory for the error word");
-        return CTBB_ERR_ALLOC;
-    }
+    int *err = copy_error_word();
+    if (!err) return CTBB_ERR_ALLOC;
     const dim3 grid((p.nx + tile_x(s.cw) - 1) / tile_x(s.cw), (p.ny + kTileY - 1) / kTileY, std::max(p.n_achunks, 1));
     return with_staged(s, [&](auto cw, auto pitch) -> int {
         constexpr int CW = decltype(cw)::value, PITCH = decltype(pitch)::value;
@@ -768,11 +686,8 @@ int launch_backproject_staged_batch(const BpParams *d_params, const unsigned *d_
                                     unsigned total, int n, int ac, int n_ac, const StagedShape &s,
                                     cudaStream_t stream)
 {
-    int *err = error_word();
-    if (!err) {
-        set_error("backproject: no pinned memory for the error word");
-        return CTBB_ERR_ALLOC;
-    }
+    int *err = copy_error_word();
+    if (!err) return CTBB_ERR_ALLOC;
     return with_staged(s, [&](auto cw, auto pitch) -> int {
         constexpr int CW = decltype(cw)::value, PITCH = decltype(pitch)::value;
         const StagedLayout lay = staged_layout(CW, s.half_bytes);
@@ -784,16 +699,6 @@ int launch_backproject_staged_batch(const BpParams *d_params, const unsigned *d_
         CTBB_CUDA_TRY(cudaGetLastError());
         return CTBB_OK;
     });
-}
-
-int staged_error_check()
-{
-    int *w = error_word();
-    if (w && *reinterpret_cast<volatile int *>(w)) {
-        set_error("backproject: a wait on a shared-memory stage ran out; the image is not valid");
-        return CTBB_ERR_CUDA;
-    }
-    return CTBB_OK;
 }
 
 }  // namespace ctbb

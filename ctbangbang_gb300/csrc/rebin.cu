@@ -28,12 +28,14 @@
 // reference's copy loops do, e.g. src/rebin_filter_cpu.cu:119-131).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
 #include "ctbb_internal.h"
 #include "cuda_util.cuh"
 #include "rebin.h"
+#include "tma.cuh"
 
 namespace ctbb {
 
@@ -232,6 +234,35 @@ int build_rebin_tables(const struct recon_metadata &mr, RebinTables *t)
         return CTBB_ERR_CONFIG;
     }
     (void)two_pi;
+    // the tiles' reads, from the taps and terms above
+    const bool two_stage = t->mode == RebinMode::kPhiFfs || t->mode == RebinMode::kBothFfs;
+    const int sides = two_stage ? (t->n_ffs == 4 ? 2 : 1) : t->n_ffs;
+    const int n_tiles = (Nos + kRebinTile - 1) / kRebinTile;
+    t->tiles.assign((size_t)sides * n_tiles, RebinTile{});
+    for (int s = 0; s < sides; ++s)
+        for (int b = 0; b < n_tiles; ++b) {
+            RebinTile &tile = t->tiles[(size_t)s * n_tiles + b];
+            int lo = N, hi = 0;
+            for (int e = 0; e < 2; ++e) {
+                tile.t_min[e] = INFINITY;
+                tile.t_max[e] = -INFINITY;
+            }
+            auto reads = [&](int ch, int e, float t_alpha) {
+                lo = std::min(lo, ch);
+                hi = std::max(hi, ch);
+                tile.t_min[e] = std::min(tile.t_min[e], t_alpha);
+                tile.t_max[e] = std::max(tile.t_max[e], t_alpha);
+            };
+            for (int c = b * kRebinTile; c < std::min(Nos, (b + 1) * kRebinTile); ++c) {
+                const AxisTap &tap = t->out_taps[(size_t)s * Nos + c];
+                for (const int i : {tap.i0, tap.i1}) {
+                    if (two_stage) reads(i >> 1, i & 1, t->focal[(size_t)(2 * s + (i & 1)) * N + (i >> 1)].t_alpha);
+                    else reads(i, 0, t->focal[(size_t)s * Nos + c].t_alpha);
+                }
+            }
+            tile.ch0 = lo & ~3;  // TMA copies start on 16 bytes
+            tile.n_ch = hi - tile.ch0 + 1;
+        }
     return CTBB_OK;
 }
 
@@ -435,6 +466,194 @@ __global__ void rebin_two_stage_kernel(RebinParams p)
     }
 }
 
+// ---- staged form ---------------------------------------------------------
+//
+// A gather of the kernels above takes 27 wavefronts of the L1 data pipe per
+// warp of outputs (81 % of its peak on a config-2 window): t_alpha moves by a
+// frame every few channels, so the 32 channels of a warp fall on four or five
+// frames of each focal spot, and one wavefront serves one of them.  Here a CTA
+// (64 output channels, kRowsPerThread raw rows, kStagedViews views of one
+// side) copies the frames its views can read -- a box of channels x rows x
+// frames per focal spot -- into shared memory by TMA (two copies) and gathers
+// from there, where frames lie a whole number of bank rounds apart and lanes of
+// consecutive channels do not collide.  Same taps, same arithmetic, same bits.
+// Small tiles: t_alpha's span over a tile adds frames to every box, so 128
+// channels (96 KB of boxes, 2 CTAs per SM) moved 3.2 GB from L2 and took 592
+// us on a config-2 window where 64 (37 KB, 6 CTAs) move 2.55 GB and take 415;
+// 32 views to a box 550, 256 threads 454; gathering 611.  What bounds it now
+// is the L2 traffic of the boxes (6.1 TB/s) beside 4.9 TB/s of HBM.
+constexpr int kStagedViews = 16;
+constexpr int kNarrowBox = 40, kWideBox = 48;  // channels of a box: a tile's, wider with a z flying focal spot
+
+struct StagedRebin {
+    const RebinTile *tiles;
+    int n_tiles, n_groups, frames;  // frames of a box
+};
+
+template <bool TWO, int CH>
+__global__ void __launch_bounds__(128) rebin_staged_kernel(RebinParams p, StagedRebin g,
+                                                           const __grid_constant__ CUtensorMap map, int *error)
+{
+    extern __shared__ __align__(128) float box[];
+    constexpr int kSpots = TWO ? 2 : 1;
+    constexpr int kFrame = kRowsPerThread * CH;  // floats between frames: a multiple of 32
+    static_assert(kFrame % 32 == 0, "frames share their banks");
+    __shared__ __align__(8) unsigned long long full;
+    const int side = blockIdx.y / g.n_groups, r0 = (blockIdx.y - side * g.n_groups) * kRowsPerThread;
+    const int v0 = p.v_begin + blockIdx.z * kStagedViews, v1 = min(v0 + kStagedViews, p.v_end);
+    const RebinTile tile = g.tiles[side * g.n_tiles + blockIdx.x];
+    const int q0 = TWO ? 2 * side : side;  // the side's first focal spot
+    // first frame of each box: one before the lowest view coordinate (its
+    // float rounding is far below a frame), inside the scan as the taps are
+    int f0[kSpots];
+#pragma unroll
+    for (int e = 0; e < kSpots; ++e) {
+        const float off = p.n_ffs == 1 ? 0.0f : p.focal_offset[q0 + e];
+        const float c = tile.t_max[e] + off + (float)(q0 + e);
+        const int lowest = (v0 + p.add) - (int)ceilf(c / (float)p.n_ffs) - 1;
+        f0[e] = min(max(lowest, 0), p.n_proj - 1);
+    }
+    const uint32_t bar = smem_address(&full);
+    if (threadIdx.x == 0) {
+        barrier_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        barrier_arrive_expect(bar, (uint32_t)(kSpots * g.frames * kFrame) * 4u);
+#pragma unroll
+        for (int e = 0; e < kSpots; ++e)
+            asm volatile(
+                "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
+                "%5}], [%6];" ::"r"(smem_address(box + e * g.frames * kFrame)),
+                "l"(reinterpret_cast<uint64_t>(&map)), "r"(tile.ch0), "r"(r0), "r"(q0 + e), "r"(f0[e]), "r"(bar)
+                : "memory");
+    }
+    __syncthreads();
+    const int c = blockIdx.x * kRebinTile + (threadIdx.x & (kRebinTile - 1));
+    const bool in = c < p.Nos;
+    // this thread's half of the views
+    constexpr int kHalf = kStagedViews / 2;
+    const int w0 = v0 + (int)(threadIdx.x / kRebinTile) * kHalf, w1 = min(w0 + kHalf, v1);
+    const int n_rows = min(kRowsPerThread, p.R_raw - r0);
+    AxisTap tap = {};
+    float ta0 = 0.0f, ta1 = 0.0f, to0 = 0.0f, to1 = 0.0f;
+    int e0 = 0, e1 = 0;  // focal spots of the two channel taps, within the side
+    const float *b0 = box, *b1 = box;
+    if (in) {
+        tap = p.taps[side * p.Nos + c];
+        if (TWO) {
+            e0 = tap.i0 & 1;
+            e1 = tap.i1 & 1;
+            ta0 = p.focal[(q0 + e0) * p.N + (tap.i0 >> 1)].t_alpha;
+            ta1 = p.focal[(q0 + e1) * p.N + (tap.i1 >> 1)].t_alpha;
+            to0 = p.focal_offset[q0 + e0];
+            to1 = p.focal_offset[q0 + e1];
+            b0 = box + (e0 ? g.frames * kFrame : 0) - (e0 ? f0[kSpots - 1] : f0[0]) * kFrame + (tap.i0 >> 1) - tile.ch0;
+            b1 = box + (e1 ? g.frames * kFrame : 0) - (e1 ? f0[kSpots - 1] : f0[0]) * kFrame + (tap.i1 >> 1) - tile.ch0;
+        } else {
+            ta0 = p.focal[side * p.Nos + c].t_alpha;
+            to0 = p.n_ffs == 1 ? 0.0f : p.focal_offset[side];
+            b0 = box - f0[0] * kFrame + tap.i0 - tile.ch0;
+            b1 = box - f0[0] * kFrame + tap.i1 - tile.ch0;
+        }
+    }
+    if (!barrier_wait(bar, 0)) {
+        *reinterpret_cast<volatile int *>(error) = 1;
+        wait_for_stray_copies();
+        return;
+    }
+    if (!in) return;
+    const bool z_ffs = TWO ? p.n_ffs == 4 : p.n_ffs == 2;
+    const size_t nos = (size_t)p.Nos;
+    const int out_first = z_ffs ? 2 * r0 + (p.reverse_rows ? 1 - side : side) : r0;
+    const size_t out_step = (z_ffs ? 2 : 1) * nos;
+    for (int v = w0; v < w1; ++v) {
+        const int proj = v + p.add;
+        int i0, i1, j0 = 0, j1 = 0;
+        float wa, wb = 0.0f;
+        if (p.split_view_coord) {
+            view_taps_split(p.n_ffs, proj, ta0, to0, q0 + e0, p.n_proj, &i0, &i1, &wa);
+            if (TWO) view_taps_split(p.n_ffs, proj, ta1, to1, q0 + e1, p.n_proj, &j0, &j1, &wb);
+        } else {
+            view_taps(focal_alpha(p.n_ffs, proj, ta0, to0, q0 + e0), p.n_proj, &i0, &i1, &wa);
+            if (TWO) view_taps(focal_alpha(p.n_ffs, proj, ta1, to1, q0 + e1), p.n_proj, &j0, &j1, &wb);
+        }
+        float *out = p.out + ((size_t)v * p.R + out_first) * nos + c;
+        const float oma = __fsub_rn(1.0f, wa), omb = __fsub_rn(1.0f, wb);
+        const float *x00 = b0 + i0 * kFrame, *x01 = b0 + i1 * kFrame;
+        const float *x10 = b1 + (TWO ? j0 : i0) * kFrame, *x11 = b1 + (TWO ? j1 : i1) * kFrame;
+#pragma unroll
+        for (int r = 0; r < kRowsPerThread; ++r) {
+            if (r >= n_rows) break;
+            const int o = r * CH;
+            float y;
+            if (TWO) {
+                const float T0 = __fadd_rn(__fmul_rn(x00[o], oma), __fmul_rn(x01[o], wa));
+                const float T1 = __fadd_rn(__fmul_rn(x10[o], omb), __fmul_rn(x11[o], wb));
+                y = __fadd_rn(__fmul_rn(T0, tap.one_minus_u), __fmul_rn(T1, tap.u));
+            } else {
+                const float t1 = __fmul_rn(__fmul_rn(x00[o], tap.one_minus_u), oma);
+                const float t2 = __fmul_rn(__fmul_rn(x10[o], tap.u), oma);
+                const float t5 = __fmul_rn(__fmul_rn(x01[o], tap.one_minus_u), wa);
+                const float t6 = __fmul_rn(__fmul_rn(x11[o], tap.u), wa);
+                y = __fadd_rn(__fadd_rn(__fadd_rn(t1, t2), t5), t6);
+            }
+            out[r * out_step] = y;
+        }
+    }
+}
+
+// Frames of the staged form's boxes, or 0 where it does not apply: rows off
+// 16-byte boundaries, a tile wider than the box, or t_alpha moving so fast
+// that two boxes do not fit beside another CTA's (few, wide channels).
+int staged_frames(const RebinTables &t, const float *d_raw, int spots, int *channels)
+{
+    if (t.n_channels % 4 != 0 || ((uintptr_t)d_raw & 15) != 0) return 0;
+    float span = 0.0f;
+    int widest = 0;
+    for (const RebinTile &tile : t.tiles) {
+        widest = std::max(widest, tile.n_ch);
+        for (int e = 0; e < spots; ++e)
+            if (tile.t_max[e] >= tile.t_min[e]) span = std::max(span, tile.t_max[e] - tile.t_min[e]);
+    }
+    if (widest > kWideBox) return 0;
+    *channels = widest <= kNarrowBox ? kNarrowBox : kWideBox;
+    // the views, t_alpha's span, and a frame of margin and the upper tap at either end
+    const float frames = (float)kStagedViews + std::ceil(span / (float)t.n_ffs) + 5.0f;
+    return frames <= 256.0f && frames * spots * kRowsPerThread * *channels * 4 <= 110 * 1024 ? (int)frames : 0;
+}
+
+int launch_rebin_staged(const RebinTables &t, const DeviceRebinTables &dt, const RebinParams &p, bool two, int frames,
+                        int channels, cudaStream_t stream)
+{
+    const cuuint64_t row = (cuuint64_t)t.n_channels * 4, frame = row * t.n_rows_raw;
+    const cuuint64_t dims[4] = {(cuuint64_t)t.n_channels, (cuuint64_t)t.n_rows_raw, (cuuint64_t)t.n_ffs,
+                                (cuuint64_t)t.n_proj};
+    const cuuint64_t strides[3] = {row, frame, frame * t.n_ffs};
+    const cuuint32_t box[4] = {(cuuint32_t)channels, kRowsPerThread, 1, (cuuint32_t)frames};
+    CUtensorMap map;
+    CTBB_TRY(tensor_map_f32(&map, p.raw, 4, dims, strides, box));
+    int *err = copy_error_word();
+    if (!err) return CTBB_ERR_ALLOC;
+    StagedRebin g;
+    g.tiles = dt.tiles;
+    g.n_tiles = (t.n_os + kRebinTile - 1) / kRebinTile;
+    g.n_groups = (t.n_rows_raw + kRowsPerThread - 1) / kRowsPerThread;
+    g.frames = frames;
+    const int sides = (int)t.tiles.size() / g.n_tiles;
+    const int chunks = (p.v_end - p.v_begin + kStagedViews - 1) / kStagedViews;
+    const size_t smem = (size_t)(two ? 2 : 1) * frames * kRowsPerThread * channels * sizeof(float);
+    const dim3 grid(g.n_tiles, g.n_groups * sides, chunks);
+    auto launch = [&](auto kernel) -> int {
+        CTBB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+        kernel<<<grid, 128, smem, stream>>>(p, g, map, err);
+        count_launch();
+        CTBB_CUDA_TRY(cudaGetLastError());
+        return CTBB_OK;
+    };
+    if (channels == kNarrowBox)
+        return two ? launch(rebin_staged_kernel<true, kNarrowBox>) : launch(rebin_staged_kernel<false, kNarrowBox>);
+    return two ? launch(rebin_staged_kernel<true, kWideBox>) : launch(rebin_staged_kernel<false, kWideBox>);
+}
+
 int rebin_frames_needed(const RebinTables &t, int v)
 {
     // view-axis coordinate of a focal spot's frame sequence: proj - t_alpha /
@@ -474,12 +693,15 @@ int launch_rebin(const RebinTables &t, const DeviceRebinTables &dt, const float 
         set_error("rebin: %d views / %d rows exceed the launch grid", t.n_views, t.n_rows_raw);
         return CTBB_ERR_ARGUMENT;
     }
+    const bool bilinear = t.mode == RebinMode::kNoFfs || t.mode == RebinMode::kZFfs;
+    int channels = 0;
+    if (const int frames = staged_frames(t, d_raw, bilinear ? 1 : 2, &channels))
+        return launch_rebin_staged(t, dt, p, !bilinear, frames, channels, stream);
     size_t n_raw = (size_t)t.n_ffs * t.n_proj * t.n_rows_raw * t.n_channels;
     size_t n_out = (size_t)t.n_views * t.n_rows * t.n_os;
     bool narrow = n_raw < ((size_t)1 << 31) && n_out < ((size_t)1 << 31);
     dim3 block(128);
     dim3 grid((t.n_os + 127) / 128, row_groups, chunks);
-    bool bilinear = t.mode == RebinMode::kNoFfs || t.mode == RebinMode::kZFfs;
     if (bilinear && narrow) rebin_bilinear_kernel<int><<<grid, block, 0, stream>>>(p);
     else if (bilinear) rebin_bilinear_kernel<size_t><<<grid, block, 0, stream>>>(p);
     else if (narrow) rebin_two_stage_kernel<int><<<grid, block, 0, stream>>>(p);
@@ -492,18 +714,20 @@ int launch_rebin(const RebinTables &t, const DeviceRebinTables &dt, const float 
 int upload_rebin_tables(const RebinTables &t, DeviceRebinTables *dt, cudaStream_t stream)
 {
     size_t nt = t.out_taps.size() * sizeof(AxisTap);
-    size_t nf = t.focal.size() * sizeof(FocalTerm);
-    if (dt->capacity < nt + nf) {
+    size_t nf = t.focal.size() * sizeof(FocalTerm), nb = t.tiles.size() * sizeof(RebinTile);
+    if (dt->capacity < nt + nf + nb) {
         if (dt->base) cudaFree(dt->base);
         dt->base = nullptr;
         dt->capacity = 0;
-        CTBB_CUDA_TRY(cudaMalloc(&dt->base, nt + nf));
-        dt->capacity = nt + nf;
+        CTBB_CUDA_TRY(cudaMalloc(&dt->base, nt + nf + nb));
+        dt->capacity = nt + nf + nb;
     }
     dt->taps = reinterpret_cast<AxisTap *>(dt->base);
     dt->focal = reinterpret_cast<FocalTerm *>(reinterpret_cast<char *>(dt->base) + nt);
     CTBB_CUDA_TRY(cudaMemcpyAsync(dt->taps, t.out_taps.data(), nt, cudaMemcpyHostToDevice, stream));
+    dt->tiles = reinterpret_cast<RebinTile *>(reinterpret_cast<char *>(dt->base) + nt + nf);
     CTBB_CUDA_TRY(cudaMemcpyAsync(dt->focal, t.focal.data(), nf, cudaMemcpyHostToDevice, stream));
+    CTBB_CUDA_TRY(cudaMemcpyAsync(dt->tiles, t.tiles.data(), nb, cudaMemcpyHostToDevice, stream));
     return CTBB_OK;
 }
 

@@ -22,6 +22,15 @@ struct FocalTerm {
     float t_alpha;
 };
 
+// What a tile of kRebinTile output channels of one side reads: its first raw
+// channel, the channels from there, and the extremes of t_alpha over them for
+// each of the side's focal spots (one or two).
+constexpr int kRebinTile = 64;
+struct RebinTile {
+    int ch0, n_ch;
+    float t_min[2], t_max[2];
+};
+
 struct RebinTables {
     RebinMode mode = RebinMode::kNoFfs;
     int n_ffs = 1, n_channels = 0, n_os = 0, n_rows_raw = 0, n_rows = 0;
@@ -33,6 +42,7 @@ struct RebinTables {
     int split_view_coord = 0;
     std::vector<AxisTap> out_taps;   // [side][n_os]
     std::vector<FocalTerm> focal;    // no/z-FFS: [side][n_os]; phi/both: [focal][n_channels]
+    std::vector<RebinTile> tiles;    // [side][tiles of the output channels]
     std::vector<float> focal_offset; // d_alpha_r * n_proj_ffs / (2 pi) per focal spot
 };
 
@@ -41,6 +51,7 @@ struct DeviceRebinTables {
     size_t capacity = 0;
     AxisTap *taps = nullptr;
     FocalTerm *focal = nullptr;
+    RebinTile *tiles = nullptr;
 };
 
 int build_rebin_tables(const struct recon_metadata &mr, RebinTables *t);
