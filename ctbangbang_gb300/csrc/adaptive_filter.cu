@@ -19,13 +19,13 @@
 // Every float operation is written as a separate rounding (__f*_rn) in the
 // reference's order, so the result equals the reference kernels evaluated
 // without fused multiply-adds.  GB300 mapping: step 1 is a CTA reduction per
-// frame, steps 2-3 one thread per frame, step 4 one warp per frame (the window
-// counts are integers, so splitting them across lanes is exact), step 5 a
-// per-frame float4 copy that lists the samples above the threshold in shared
-// memory and smooths them after the copy (rows of a multiple of 4 channels;
-// otherwise a shared-memory tiled stencil).  Every step takes a frame range,
-// so a window whose frames arrive in order can be filtered as they come
-// (AfStream).
+// frame that copies the frame on the way, steps 2-3 one thread per frame, step
+// 4 one warp per frame (the window counts are integers, so splitting them
+// across lanes is exact), step 5 reads the frames again that hold a sample
+// above their threshold and smooths those samples.  The window is so moved once
+// (read and written, the HBM bound); copying after the thresholds reads it
+// twice.  Every step takes a frame range, so a window whose frames arrive in
+// order can be filtered as they come (AfStream).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -51,6 +51,7 @@ struct AfParams {
     const float *raw;
     float *out;
     float *sup, *smooth, *ecc, *pmax, *pmin, *thr;
+    float *sup_out;  // maxima to write (null: they are given)
     int P, R, N;
     int n_proj_ffs;
     int n_avg, avg_offset;
@@ -59,29 +60,73 @@ struct AfParams {
     int f0, f1;  // frames this launch writes: [f0, f1) of the window [0, P)
 };
 
-__global__ void af_sup_kernel(AfParams p)
+// Groups of four consecutive samples of a frame; VEC: 16-byte accesses (whole
+// groups, aligned frames).  Samples past the frame's end read 0, which no
+// threshold lies below.
+template <bool VEC>
+__device__ __forceinline__ float4 load_group(const float *src, int i, int n)
 {
-    int proj = p.f0 + blockIdx.x;
-    size_t frame = (size_t)p.R * p.N;
-    const float *src = p.raw + (size_t)proj * frame;
-    float m = 0.0f;
-    if ((frame & 3) == 0) {  // frames start 16-byte aligned: float4 loads
-        const float4 *s4 = reinterpret_cast<const float4 *>(src);
-        for (size_t i = threadIdx.x; i < frame / 4; i += blockDim.x) {
-            float4 v = __ldg(s4 + i);
-            m = fmaxf(fmaxf(m, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
-        }
+    if constexpr (VEC) return __ldg(reinterpret_cast<const float4 *>(src) + i);
+    float4 v;
+    v.x = __ldg(src + 4 * i);
+    v.y = 4 * i + 1 < n ? __ldg(src + 4 * i + 1) : 0.0f;
+    v.z = 4 * i + 2 < n ? __ldg(src + 4 * i + 2) : 0.0f;
+    v.w = 4 * i + 3 < n ? __ldg(src + 4 * i + 3) : 0.0f;
+    return v;
+}
+
+template <bool VEC>
+__device__ __forceinline__ void store_group(float *dst, int i, int n, float4 v)
+{
+    if constexpr (VEC) {
+        reinterpret_cast<float4 *>(dst)[i] = v;
     } else {
-        for (size_t i = threadIdx.x; i < frame; i += blockDim.x) m = fmaxf(m, src[i]);
+        dst[4 * i] = v.x;
+        if (4 * i + 1 < n) dst[4 * i + 1] = v.y;
+        if (4 * i + 2 < n) dst[4 * i + 2] = v.z;
+        if (4 * i + 3 < n) dst[4 * i + 3] = v.w;
+    }
+}
+
+// Step 1, and the copy of every sample that step 5 does not change: one CTA
+// per frame, last frame first (the rebinning starts with the first, which L2
+// then still holds), kCopyUnroll groups in flight per thread.  Bound by HBM:
+// 11 264 frames of 736 x 32 (1.06 GB each way) in 300 us, 7.1 TB/s.  The maxima
+// and the copy as separate passes: 146 + 365 us.  Eight CTAs per SM, unrolls of
+// 2 and 8 and streaming loads or stores are within 3 % or slower.
+constexpr int kCopyUnroll = 4;
+
+template <bool VEC>
+__global__ void __launch_bounds__(256, 4) af_copy_kernel(AfParams p)
+{
+    const int proj = p.f1 - 1 - (int)blockIdx.x;
+    const size_t frame = (size_t)p.R * p.N;
+    const float *src = p.raw + (size_t)proj * frame;
+    float *dst = p.out + (size_t)proj * frame;
+    const int n = (int)frame, n4 = (n + 3) / 4;
+    float m = 0.0f;
+    for (int i0 = threadIdx.x; i0 < n4; i0 += kCopyUnroll * 256) {
+        float4 v[kCopyUnroll];
+#pragma unroll
+        for (int u = 0; u < kCopyUnroll; ++u) {
+            const int i = i0 + u * 256;
+            v[u] = i < n4 ? load_group<VEC>(src, i, n) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int u = 0; u < kCopyUnroll; ++u) {
+            const int i = i0 + u * 256;
+            if (i < n4) store_group<VEC>(dst, i, n, v[u]);
+            m = fmaxf(fmaxf(m, fmaxf(v[u].x, v[u].y)), fmaxf(v[u].z, v[u].w));
+        }
     }
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    __shared__ float red[32];
+    __shared__ float red[8];
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     if (threadIdx.x < 32) {
-        m = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0f;
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (threadIdx.x == 0) p.sup[proj] = m;
+        m = threadIdx.x < 8 ? red[threadIdx.x] : 0.0f;
+        for (int o = 4; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (threadIdx.x == 0 && p.sup_out) p.sup_out[proj] = m;
     }
 }
 
@@ -278,165 +323,138 @@ __global__ void __launch_bounds__(256) af_threshold_kernel(AfParams p)
     if (lane == 0) p.thr[proj] = T;
 }
 
-// Stencil tile: TP frames x TR rows x TC channels of output per CTA.
-constexpr int TP = 4, TR = 8, TC = 32;
-constexpr int SP = TP + 4, SR = TR + 4, SC = TC + 4;
+// 5x5x5 triangle smoothing of up to kWarpSamples listed samples (frame, sample
+// of the frame) by a warp, taps added in the reference's order (channel, row,
+// frame).  The lanes fetch all taps at once into shared memory, one tap of
+// every sample per kWarpSamples lanes, and a lane then adds its sample's; a
+// thread that fetched its own sample's taps waited for them five times, and a
+// list is often shorter than a warp.  A tap out of range counts as 0, which
+// leaves the sum as it is; norm is the exact integer sum of the weights in
+// range.
+constexpr int kWarpSamples = 4;
 
-__global__ void __launch_bounds__(256) af_filter_kernel(AfParams p)
+__device__ __forceinline__ void smooth_samples(const AfParams &p, const int2 *list, int n, float *taps)
 {
-    __shared__ float tile[SP][SR][SC];
-    int c0 = blockIdx.x * TC, r0 = blockIdx.y * TR, p0 = p.f0 + blockIdx.z * TP;
-    size_t frame = (size_t)p.R * p.N;
-    for (int t = threadIdx.x; t < SP * SR * SC; t += blockDim.x) {
-        int sc = t % SC, sr = (t / SC) % SR, sp = t / (SC * SR);
-        int gc = c0 + sc - 2, gr = r0 + sr - 2, gp = p0 + sp - 2;
-        float v = 0.0f;
-        if (gc >= 0 && gc < p.N && gr >= 0 && gr < p.R && gp >= 0 && gp < p.P)
-            v = __ldg(p.raw + (size_t)gp * frame + (size_t)gr * p.N + gc);
-        tile[sp][sr][sc] = v;
+    const int lane = threadIdx.x & 31, s = lane % kWarpSamples;
+    const size_t frame = (size_t)p.R * p.N;
+    const int2 at = list[min(s, n - 1)];
+    const int gp = at.x, gr = at.y / p.N, gc = at.y - gr * p.N;
+    constexpr int kTapLanes = 32 / kWarpSamples, kFetch = (125 + kTapLanes - 1) / kTapLanes;
+    float x[kFetch];
+#pragma unroll
+    for (int m = 0; m < kFetch; ++m) {
+        const int tap = lane / kWarpSamples + kTapLanes * m;
+        const int c = gc + tap / 25 - 2, r = gr + tap / 5 % 5 - 2, f = gp + tap % 5 - 2;
+        const bool in = tap < 125 && c >= 0 && c < p.N && r >= 0 && r < p.R && f >= 0 && f < p.P;
+        x[m] = in ? __ldg(p.raw + (size_t)f * frame + (size_t)r * p.N + c) : 0.0f;
     }
-    __syncthreads();
-    for (int t = threadIdx.x; t < TP * TR * TC; t += blockDim.x) {
-        int lc = t % TC, lr = (t / TC) % TR, lp = t / (TC * TR);
-        int gc = c0 + lc, gr = r0 + lr, gp = p0 + lp;
-        if (gc >= p.N || gr >= p.R || gp >= p.f1) continue;
-        float x = tile[lp + 2][lr + 2][lc + 2];
-        float T = p.thr[gp];
-        float y = x;
-        if (x > T) {
-            // norm = sum of in-bounds weights: an exact integer, independent of order
-            int ni = 0, nj = 0, nk = 0, si = 0, sj = 0, sk = 0;
-            for (int d = 0; d < 5; ++d) {
-                if (gc + d - 2 >= 0 && gc + d - 2 < p.N) { ni++; si += tri1(d); }
-                if (gr + d - 2 >= 0 && gr + d - 2 < p.R) { nj++; sj += tri1(d); }
-                if (gp + d - 2 >= 0 && gp + d - 2 < p.P) { nk++; sk += tri1(d); }
-            }
-            float norm = (float)(nj * nk * si + ni * nk * sj + ni * nj * sk + ni * nj * nk);
-            // taps in the reference's order (channel, row, frame); the weights
-            // are compile-time constants of the fully unrolled loops
-            float val = 0.0f;
+    __syncwarp();
 #pragma unroll
-            for (int ii = 0; ii < 5; ii++)
+    for (int m = 0; m < kFetch; ++m)
+        if (lane / kWarpSamples + kTapLanes * m < 125) taps[lane + 32 * m] = x[m];
+    __syncwarp();
+    if (lane < min(n, kWarpSamples)) {
+        int ni = 0, nj = 0, nk = 0, si = 0, sj = 0, sk = 0;
 #pragma unroll
-                for (int jj = 0; jj < 5; jj++)
-#pragma unroll
-                    for (int kk = 0; kk < 5; kk++)
-                        val = __fadd_rn(val, __fmul_rn(tile[lp + kk][lr + jj][lc + ii],
-                                                       (float)(tri1(ii) + tri1(jj) + tri1(kk) + 1)));
-            y = __fmul_rn(__fdiv_rn(1.0f, norm), val);
+        for (int d = 0; d < 5; ++d) {
+            if (gc + d - 2 >= 0 && gc + d - 2 < p.N) { ni++; si += tri1(d); }
+            if (gr + d - 2 >= 0 && gr + d - 2 < p.R) { nj++; sj += tri1(d); }
+            if (gp + d - 2 >= 0 && gp + d - 2 < p.P) { nk++; sk += tri1(d); }
         }
-        p.out[(size_t)gp * frame + (size_t)gr * p.N + gc] = y;
+        const float norm = (float)(nj * nk * si + ni * nk * sj + ni * nj * sk + ni * nj * nk);
+        float val = 0.0f;
+#pragma unroll
+        for (int t = 0; t < 125; ++t)
+            val = __fadd_rn(val, __fmul_rn(taps[kWarpSamples * t + lane],
+                                           (float)(tri1(t / 25) + tri1(t / 5 % 5) + tri1(t % 5) + 1)));
+        p.out[(size_t)gp * frame + at.y] = __fmul_rn(__fdiv_rn(1.0f, norm), val);
     }
 }
 
-// 5x5x5 triangle smoothing of one sample, taps in the reference's order
-// (channel, row, frame) with out-of-range taps skipped; norm is the exact
-// integer sum of the in-range weights.
-__device__ __noinline__ float smooth_sample(const AfParams &p, int gp, int gr, int gc)
-{
-    size_t frame = (size_t)p.R * p.N;
-    int ni = 0, nj = 0, nk = 0, si = 0, sj = 0, sk = 0;
-#pragma unroll
-    for (int d = 0; d < 5; ++d) {
-        if (gc + d - 2 >= 0 && gc + d - 2 < p.N) { ni++; si += tri1(d); }
-        if (gr + d - 2 >= 0 && gr + d - 2 < p.R) { nj++; sj += tri1(d); }
-        if (gp + d - 2 >= 0 && gp + d - 2 < p.P) { nk++; sk += tri1(d); }
-    }
-    float norm = (float)(nj * nk * si + ni * nk * sj + ni * nj * sk + ni * nj * nk);
-    float val = 0.0f;
-#pragma unroll 1
-    for (int ii = 0; ii < 5; ii++) {
-        int c = gc + ii - 2;
-        if (c < 0 || c >= p.N) continue;
-        // the channel's 25 taps are all fetched before the first is added (a
-        // list is often shorter than a warp, its latency the whole cost)
-        float x[5][5];
-#pragma unroll
-        for (int jj = 0; jj < 5; jj++)
-#pragma unroll
-            for (int kk = 0; kk < 5; kk++) {
-                const int r = gr + jj - 2, f = gp + kk - 2;
-                const bool in = r >= 0 && r < p.R && f >= 0 && f < p.P;
-                x[jj][kk] = in ? __ldg(p.raw + (size_t)f * frame + (size_t)r * p.N + c) : 0.0f;
-            }
-#pragma unroll
-        for (int jj = 0; jj < 5; jj++)
-#pragma unroll
-            for (int kk = 0; kk < 5; kk++) {
-                const int r = gr + jj - 2, f = gp + kk - 2;
-                if (r < 0 || r >= p.R || f < 0 || f >= p.P) continue;
-                val = __fadd_rn(val, __fmul_rn(x[jj][kk], (float)(tri1(ii) + tri1(jj) + tri1(kk) + 1)));
-            }
-    }
-    return __fmul_rn(__fdiv_rn(1.0f, norm), val);
-}
+// Step 5, on a copy of the frames (af_copy_kernel): only frames whose maximum
+// exceeds their threshold are read again (thresholds lie between means of
+// maxima, so they are never negative), one in twenty at strength 1.  They come
+// in short runs, so a frame is cut into kParts parts, and each CTA serves one
+// part of every `lanes`-th frame: it lists the samples above the threshold in
+// shared memory, over all its frames, and smooths them together, or earlier
+// when the list runs full.  Bound by the waits of its chain (thresholds, four
+// rounds of loads at a time, taps): 42 us for the window above, where a CTA per
+// frame with a thread per listed sample took 69 us; 4 or 16 parts take 2 %
+// longer for the call, 8 rounds at a time 4 %.
+constexpr int kParts = 8;
+constexpr int kAhead = 4;
+constexpr int kListRoom = 4 * 256;  // samples a round can add
+constexpr int kSmoothListMax = 2 * kListRoom;
+constexpr int kFilterCtas = 2;
 
-// Streaming form for rows of a multiple of 4 channels: one CTA per frame
-// copies the frame with float4 loads/stores and notes the samples above the
-// frame's threshold -- about 1e-4 of them on clinical-size scans -- in a
-// shared-memory list; after the copy the CTA smooths the listed samples (or,
-// when the list overflowed, every sample above the threshold again).  The
-// copy loop holds no call, so it runs at copy speed.  Same arithmetic, same
-// result as the tiled form.
-constexpr int kSmoothListMax = 1024;
-
-__global__ void __launch_bounds__(256, 4) af_filter_stream_kernel(AfParams p)
+template <bool VEC>
+__global__ void __launch_bounds__(256, kFilterCtas) af_filter_kernel(AfParams p)
 {
-    __shared__ int list[kSmoothListMax];
-    __shared__ int n_list;
-    // last frame first: the end of the range is what the maxima's pass left in
-    // L2, and its beginning is what the rebinning reads first
-    int gp = p.f1 - 1 - (int)blockIdx.x;
-    size_t frame = (size_t)p.R * p.N;
-    const float4 *src = reinterpret_cast<const float4 *>(p.raw + (size_t)gp * frame);
-    float4 *dst = reinterpret_cast<float4 *>(p.out + (size_t)gp * frame);
-    float *dst1 = p.out + (size_t)gp * frame;
-    const float T = __ldg(p.thr + gp);
-    const int n4 = (int)(frame / 4);
+    __shared__ int2 list[kSmoothListMax];
+    __shared__ float taps[8][125 * kWarpSamples];
+    __shared__ int active[256];
+    __shared__ float active_thr[256];
+    __shared__ int n_list, n_active;
+    const int part = blockIdx.x % kParts, lanes = gridDim.x / kParts;
+    const size_t frame = (size_t)p.R * p.N;
+    const int n_frame = (int)frame, n4 = (n_frame + 3) / 4;
+    const int g0 = (int)((long long)part * n4 / kParts), g1 = (int)((long long)(part + 1) * n4 / kParts);
+    auto smooth_listed = [&] {
+        const int n = n_list;
+        for (int j = (int)threadIdx.x / 32 * kWarpSamples; j < n; j += 8 * kWarpSamples)
+            smooth_samples(p, list + j, n - j, taps[threadIdx.x / 32]);
+    };
     if (threadIdx.x == 0) n_list = 0;
-    __syncthreads();
-    // kUnroll independent 16-byte loads in flight per thread
-    constexpr int kUnroll = 4;
-    for (int i0 = threadIdx.x; i0 < n4; i0 += kUnroll * blockDim.x) {
-        float4 v[kUnroll];
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            int i = i0 + u * blockDim.x;
-            if (i < n4) v[u] = __ldg(src + i);
+    for (int first = p.f0 + (int)blockIdx.x / kParts; first < p.f1; first += 256 * lanes) {
+        if (threadIdx.x == 0) n_active = 0;
+        __syncthreads();
+        const int f = first + (int)threadIdx.x * lanes;
+        const float T = f < p.f1 ? __ldg(p.thr + f) : 0.0f;
+        if (f < p.f1 && __ldg(p.sup + f) > T) {
+            const int slot = atomicAdd(&n_active, 1);
+            active[slot] = f;
+            active_thr[slot] = T;
         }
+        __syncthreads();
+        const int n = n_active;
+        // rounds of 256 groups, the loads of kAhead of them in flight
+        const int rounds = (g1 - g0 + 255) / 256;
+        for (int w0 = 0; w0 < n * rounds; w0 += kAhead) {
+            float4 v[kAhead];
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            int i = i0 + u * blockDim.x;
-            if (i >= n4) break;
-            dst[i] = v[u];
-            if (v[u].x > T || v[u].y > T || v[u].z > T || v[u].w > T) {
-                float c[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+            for (int u = 0; u < kAhead; ++u) {
+                const int a = (w0 + u) / rounds, i = g0 + (w0 + u - a * rounds) * 256 + (int)threadIdx.x;
+                v[u] = a < n && i < g1 ? load_group<VEC>(p.raw + (size_t)active[a] * frame, i, n_frame)
+                                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (c[e] > T) {
-                        int slot = atomicAdd(&n_list, 1);
-                        if (slot < kSmoothListMax) list[slot] = 4 * i + e;
-                    }
+            for (int u = 0; u < kAhead; ++u) {
+                const int a = (w0 + u) / rounds, i = g0 + (w0 + u - a * rounds) * 256 + (int)threadIdx.x;
+                if (a >= n) break;
+                const float T = active_thr[a];
+                int last = 0;
+                if (v[u].x > T || v[u].y > T || v[u].z > T || v[u].w > T) {
+                    const float c[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (c[e] > T) {
+                            last = atomicAdd(&n_list, 1);
+                            list[last] = make_int2(active[a], 4 * i + e);
+                        }
+                }
+                // a slot of the list's second half was taken: the next round may not fit
+                if (__syncthreads_or(last >= kListRoom)) {
+                    smooth_listed();
+                    __syncthreads();
+                    if (threadIdx.x == 0) n_list = 0;
+                    __syncthreads();
+                }
             }
         }
+        __syncthreads();  // `active` and its count are read before they are written again
     }
     __syncthreads();
-    const int n = n_list;
-    if (n <= kSmoothListMax) {
-        for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            int e = list[j];
-            int gr = e / p.N, gc = e - gr * p.N;
-            dst1[e] = smooth_sample(p, gp, gr, gc);
-        }
-    } else {
-        const float *src1 = p.raw + (size_t)gp * frame;
-        for (int e = threadIdx.x; e < (int)frame; e += blockDim.x) {
-            if (__ldg(src1 + e) > T) {
-                int gr = e / p.N, gc = e - gr * p.N;
-                dst1[e] = smooth_sample(p, gp, gr, gc);
-            }
-        }
-    }
+    smooth_listed();
 }
 
 // One thread per frame of the window: can this window's filtered frame
@@ -491,6 +509,7 @@ int af_params(const struct recon_metadata &mr, const float *d_in, float *d_out, 
     p.n_range = n_range;
     p.range_offset = (int)floorf((float)(n_range / 2));
     p.strength = mr.rp.adaptive_filtration_s;
+    p.sup_out = nullptr;
     p.f0 = 0;
     p.f1 = p.P;
     if (p.P <= 0 || p.R <= 0 || p.N <= 0) {
@@ -500,20 +519,25 @@ int af_params(const struct recon_metadata &mr, const float *d_in, float *d_out, 
     return CTBB_OK;
 }
 
-// The five steps over frame ranges: maxima of [sup0, sup1), moving means of
-// [smooth0, smooth1), eccentricity, threshold and smoothing of [out0, out1)
-// (eccentricity and threshold only with `thresholds`, smoothing only with
-// `output`).  Each range may be empty; a step reads the earlier steps'
-// results of the frames its windows cover, which the caller has launched
-// before.
-int af_launch(AfParams p, int sup0, int sup1, int smooth0, int smooth1, int out0, int out1, cudaStream_t stream,
-              bool thresholds = true, bool output = true)
+// The five steps over frame ranges: maxima (and the copy) of [sup0, sup1),
+// moving means of [smooth0, smooth1), eccentricity and threshold of [thr0,
+// thr1), smoothing of [out0, out1).  `copied`: the frames of the last range
+// went through the first step with this p.out; otherwise the last step copies
+// them too.  Each range may be empty; a step reads the earlier steps' results
+// of the frames its windows cover, which the caller has launched before.
+int af_launch(AfParams p, int sup0, int sup1, int smooth0, int smooth1, int thr0, int thr1, int out0, int out1,
+              bool copied, cudaStream_t stream)
 {
     int launches = 0;
+    // frames start 16-byte aligned: whole groups of four
+    const bool vec = (size_t)p.R * p.N % 4 == 0 &&
+                     (reinterpret_cast<uintptr_t>(p.raw) | reinterpret_cast<uintptr_t>(p.out)) % 16 == 0;
     if (sup1 > sup0) {
         p.f0 = sup0;
         p.f1 = sup1;
-        af_sup_kernel<<<sup1 - sup0, 256, 0, stream>>>(p);
+        p.sup_out = p.sup;
+        if (vec) af_copy_kernel<true><<<sup1 - sup0, 256, 0, stream>>>(p);
+        else af_copy_kernel<false><<<sup1 - sup0, 256, 0, stream>>>(p);
         ++launches;
     }
     if (smooth1 > smooth0) {
@@ -522,10 +546,10 @@ int af_launch(AfParams p, int sup0, int sup1, int smooth0, int smooth1, int out0
         af_smooth_kernel<<<(smooth1 - smooth0 + 127) / 128, 128, (size_t)(127 + p.n_avg) * sizeof(float), stream>>>(p);
         ++launches;
     }
-    if (out1 > out0 && thresholds) {
-        int n = out1 - out0;
-        p.f0 = out0;
-        p.f1 = out1;
+    if (thr1 > thr0) {
+        int n = thr1 - thr0;
+        p.f0 = thr0;
+        p.f1 = thr1;
         if (ecc_smem(p.n_range) <= kEccSmem)
             af_ecc_kernel<<<(n + kEccFrames - 1) / kEccFrames, kEccFrames, ecc_smem(p.n_range), stream>>>(p);
         else
@@ -538,20 +562,19 @@ int af_launch(AfParams p, int sup0, int sup1, int smooth0, int smooth1, int out0
         else af_threshold_kernel<0><<<ctas, 256, 0, stream>>>(p);
         launches += 2;
     }
-    if (out1 > out0 && output) {
-        int n = out1 - out0;
+    if (out1 > out0) {
+        const int n = out1 - out0;
         p.f0 = out0;
         p.f1 = out1;
-        if (p.N % 4 == 0) {
-            af_filter_stream_kernel<<<n, 256, 0, stream>>>(p);
-        } else {
-            dim3 grid((p.N + TC - 1) / TC, (p.R + TR - 1) / TR, (n + TP - 1) / TP);
-            if (grid.z > 65535) {
-                set_error("adaptive filter: %d frames exceed the launch grid", n);
-                return CTBB_ERR_ARGUMENT;
-            }
-            af_filter_kernel<<<grid, 256, 0, stream>>>(p);
+        if (!copied) {
+            p.sup_out = nullptr;
+            if (vec) af_copy_kernel<true><<<n, 256, 0, stream>>>(p);
+            else af_copy_kernel<false><<<n, 256, 0, stream>>>(p);
+            ++launches;
         }
+        const int grid = kParts * std::min(n, num_sms() * kFilterCtas / kParts);
+        if (vec) af_filter_kernel<true><<<grid, 256, 0, stream>>>(p);
+        else af_filter_kernel<false><<<grid, 256, 0, stream>>>(p);
         launches += 1;
     }
     count_launch(launches);
@@ -566,7 +589,7 @@ int launch_adaptive_filter(const struct recon_metadata &mr, const float *d_in, f
 {
     AfParams p;
     CTBB_TRY(af_params(mr, d_in, d_out, d_scratch, &p));
-    return af_launch(p, 0, p.P, 0, p.P, 0, p.P, stream);
+    return af_launch(p, 0, p.P, 0, p.P, 0, p.P, 0, p.P, true, stream);
 }
 
 int adaptive_filter_edge_reach(const struct recon_metadata &mr)
@@ -585,8 +608,8 @@ int launch_adaptive_filter_ends_thresholds(const struct recon_metadata &mr, cons
     p.sup = const_cast<float *>(d_sup);  // read only: no maxima are launched
     fa = std::min(std::max(fa, 0), p.P);
     fb = std::min(std::max(fb, fa), p.P);
-    CTBB_TRY(af_launch(p, 0, 0, 0, p.P, 0, fa, stream, true, false));
-    return af_launch(p, 0, 0, 0, 0, fb, p.P, stream, true, false);
+    CTBB_TRY(af_launch(p, 0, 0, 0, p.P, 0, fa, 0, 0, false, stream));
+    return af_launch(p, 0, 0, 0, 0, fb, p.P, 0, 0, false, stream);
 }
 
 int launch_adaptive_filter_dirty(const struct recon_metadata &mr, const float *d_sup, const float *d_thr_union,
@@ -613,7 +636,7 @@ int launch_adaptive_filter_output(const struct recon_metadata &mr, const float *
     p.sup = const_cast<float *>(d_sup);
     f0 = std::min(std::max(f0, 0), p.P);
     f1 = std::min(std::max(f1, f0), p.P);
-    return af_launch(p, 0, 0, 0, 0, f0, f1, stream, false, true);
+    return af_launch(p, 0, 0, 0, 0, 0, 0, f0, f1, false, stream);
 }
 
 AfStream::AfStream(const struct recon_metadata &mr) : P((int)mr.ri.n_proj_pull)
@@ -641,7 +664,8 @@ int AfStream::advance(const struct recon_metadata &mr, const float *d_in, float 
     int finished = all ? P : std::max(0, std::min(smoothed - range_reach, arrived - 2));
     smoothed = std::max(smoothed, n_smoothed);
     finished = std::max(finished, n_filtered);
-    CTBB_TRY(af_launch(p, n_sup, arrived, n_smoothed, smoothed, n_filtered, finished, stream));
+    CTBB_TRY(af_launch(p, n_sup, arrived, n_smoothed, smoothed, n_filtered, finished, n_filtered, finished, true,
+                       stream));
     n_sup = std::max(n_sup, arrived);
     n_smoothed = smoothed;
     n_filtered = finished;

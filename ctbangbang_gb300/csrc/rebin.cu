@@ -1,6 +1,6 @@
 // rebin.cu -- flying-focal-spot split + fan-to-parallel rebinning.
 //
-// One fused gather kernel per FFS mode replaces the reference's reshape /
+// One fused kernel per FFS mode replaces the reference's reshape /
 // azimuthal / radial kernel chain (src/rebin_filter.cu:58-912) and the CPU twin
 // it must match (src/rebin_filter_cpu.cu:95-645):
 //
@@ -19,9 +19,13 @@
 // that no multiply-add is fused.  The unfiltered result is therefore bit-exact
 // with the reference CPU path compiled without FMA contraction.
 //
-// A thread covers one output channel, 8 views and 4 raw rows: the view-axis
-// taps of a (channel, view) are computed once for its rows.  A launch may
-// cover a range of views (the streamed whole-scan path).
+// Two forms with the same taps and arithmetic.  The staged one copies the
+// frames that a tile of output channels and views can read to shared memory by
+// TMA; the gathering one (channel counts that are not a multiple of 4, raw
+// pointers off 16 bytes, tiles too wide for the box) reads them through L1.  In
+// both a thread covers one output channel and 4 raw rows, so the view-axis taps
+// of a (channel, view) are computed once for its rows.  A launch may cover a
+// range of views (the streamed whole-scan path).
 //
 // Output layout: rebin[view][out_row][channel_os], views = n_proj/n_ffs -
 // 2*add_projections (the leading add_projections views are dropped, as the
