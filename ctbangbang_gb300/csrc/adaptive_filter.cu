@@ -227,51 +227,82 @@ __global__ void af_ecc_long_kernel(AfParams p)
     write_ecc(p, proj, vmax, vmin);
 }
 
-// One warp per frame: the bisection of find_thresholds with the window count
-// of rhs() (include/preprocessing.cuh:32-62), an exact integer, split over the
-// lanes.  NV > 0: a lane keeps its NV values of the window in registers, so
-// that a step of the bisection reads nothing (a value beyond the window is
-// -inf, never above a threshold); NV = 0: windows of more than 2560 frames
-// are read again each step.  A value at or below the lower bound is never
-// counted again and one above the upper bound always is: once at most 256
-// values lie between, only those are kept and compared, 8 to a lane (after
-// three or four of the up to 21 steps on a window of 2305).  11 264 frames of
-// 2305: 101 us read again each step, 89 us all from registers, 70 us so.
-constexpr int kFew = 8;  // values per lane once few are left
+// Step 4: the reference's bisection, one warp per frame.  STAGED: the window of
+// a CTA's frames is in shared memory with the extremes of each 32 means, so a
+// count above T reads only the few chunks that T cuts through -- the means are
+// 18 degree averages, so a chunk is narrow -- and once 256 values lie between
+// the bounds they move to registers.  11 264 frames of 2305: 70 us with the
+// window in registers and every count over all of it, 43 us so (4446 and 3250
+// instructions a frame, and the chain of a bisection's steps).  Otherwise a
+// window of up to 256 means is in registers from the start (192 views a turn:
+// 2 us faster than staged), and one beyond kThrSmem counts from global memory.
+constexpr int kThrFrames = 8;  // frames (warps) per CTA
+constexpr int kFew = 8;        // values per lane once few are left
+constexpr size_t kThrSmem = 48 * 1024;
 
-template <int NV>
-__global__ void __launch_bounds__(256) af_threshold_kernel(AfParams p)
+__host__ __device__ constexpr int thr_chunks(int n_range) { return (n_range + kThrFrames - 1 + 31) / 32; }
+__host__ __device__ constexpr size_t thr_smem(int n_range)
 {
-    __shared__ float few[8][32 * kFew];
-    const int lane = threadIdx.x & 31;
-    const int proj = p.f0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (proj >= p.f1) return;
-    // the window, cut at the scan's ends
+    return sizeof(float) * ((size_t)thr_chunks(n_range) * (32 + 2) + kThrFrames * 32 * kFew);
+}
+
+template <bool STAGED>
+__global__ void __launch_bounds__(32 * kThrFrames) af_threshold_kernel(AfParams p)
+{
+    extern __shared__ float win[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = p.f0 + (int)blockIdx.x * kThrFrames, proj = first + warp;
+    // the CTA's window and this frame's, cut at the scan's ends
+    const int cta_begin = max(first - p.range_offset, 0);
     const int begin = max(proj - p.range_offset, 0);
     const int numel = min(proj - p.range_offset + p.n_range, p.P) - begin;
-    const float *win = p.smooth + begin;
-    float v[NV > 0 ? NV : 1];
-    if constexpr (NV > 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) v[k] = lane + 32 * k < numel ? win[lane + 32 * k] : -INFINITY;
+    float *lo = win + 32 * thr_chunks(p.n_range), *hi = lo + thr_chunks(p.n_range);
+    float *kept = hi + thr_chunks(p.n_range) + warp * (32 * kFew);
+    if (STAGED) {
+        const int last = min(first + kThrFrames, p.f1) - 1;
+        const int len = min(last - p.range_offset + p.n_range, p.P) - cta_begin;
+        for (int c = warp; 32 * c < len; c += kThrFrames) {
+            const float v = 32 * c + lane < len ? p.smooth[cta_begin + 32 * c + lane] : 0.0f;
+            win[32 * c + lane] = v;
+            // means are never negative: their bits order as they do
+            const unsigned least = __reduce_min_sync(0xffffffffu, __float_as_uint(v));
+            const unsigned most = __reduce_max_sync(0xffffffffu, __float_as_uint(v));
+            if (lane == 0) {
+                lo[c] = __uint_as_float(least);
+                hi[c] = __uint_as_float(most);
+            }
+        }
+        __syncthreads();
     }
+    if (proj >= p.f1) return;
+    const int w0 = begin - cta_begin, w1 = w0 + numel;  // this frame's window in `win`
+    const int c1 = (w1 + 31) / 32;
     int above = 0;  // values no longer kept that are above every further threshold
     bool is_few = false;
+    float v[kFew];  // a value not kept is -inf, never above a threshold
+    if (!STAGED && numel <= 32 * kFew) {
+#pragma unroll
+        for (int k = 0; k < kFew; ++k) v[k] = lane + 32 * k < numel ? p.smooth[begin + lane + 32 * k] : -INFINITY;
+        is_few = true;
+    }
     auto count = [&](float T) {
         int n = 0;
-        if (is_few || (NV > 0 && NV <= kFew)) {
+        if (is_few) {
 #pragma unroll
-            for (int k = 0; k < (NV > 0 ? min(NV, kFew) : 1); ++k) n += v[k] > T ? 1 : 0;
-        } else if constexpr (NV > 0) {
-            int m = 0;
-#pragma unroll
-            for (int k = 0; k < NV; k += 2) {
-                n += v[k] > T ? 1 : 0;
-                m += v[k + 1] > T ? 1 : 0;
+            for (int k = 0; k < kFew; ++k) n += v[k] > T ? 1 : 0;
+        } else if (STAGED) {
+            for (int base = w0 / 32; base < c1; base += 32) {
+                const int c = base + lane;
+                const bool some = c < c1 && hi[min(c, c1 - 1)] > T;
+                const bool all = some && lo[c] > T && 32 * c >= w0 && 32 * c + 32 <= w1;
+                n += all ? 32 : 0;
+                for (unsigned m = __ballot_sync(0xffffffffu, some && !all); m; m &= m - 1) {
+                    const int i = 32 * (base + __ffs(m) - 1) + lane;
+                    n += i >= w0 && i < w1 && win[i] > T ? 1 : 0;
+                }
             }
-            n += m;
         } else {
-            for (int i = lane; i < numel; i += 32) n += win[i] > T ? 1 : 0;
+            for (int i = lane; i < numel; i += 32) n += p.smooth[begin + i] > T ? 1 : 0;
         }
         return __reduce_add_sync(0xffffffffu, n) + above;
     };
@@ -298,23 +329,25 @@ __global__ void __launch_bounds__(256) af_threshold_kernel(AfParams p)
         } else {
             break;
         }
-        if constexpr (NV > kFew) {
-            if (!is_few && n_lower - n_upper <= 32 * kFew) {
-                float *kept = few[threadIdx.x >> 5];
-                int at = 0;
-#pragma unroll
-                for (int k = 0; k < NV; ++k) {
-                    const bool keep = v[k] > lower && v[k] <= upper;
+        if (STAGED && !is_few && n_lower - n_upper <= 32 * kFew) {
+            int at = 0;
+            for (int base = w0 / 32; base < c1; base += 32) {
+                const int c = base + lane;
+                const bool some = c < c1 && hi[min(c, c1 - 1)] > lower && lo[min(c, c1 - 1)] <= upper;
+                for (unsigned m = __ballot_sync(0xffffffffu, some); m; m &= m - 1) {
+                    const int i = 32 * (base + __ffs(m) - 1) + lane;
+                    const float x = win[i];
+                    const bool keep = i >= w0 && i < w1 && x > lower && x <= upper;
                     const unsigned who = __ballot_sync(0xffffffffu, keep);
-                    if (keep) kept[at + __popc(who & ((1u << lane) - 1u))] = v[k];
+                    if (keep) kept[at + __popc(who & ((1u << lane) - 1u))] = x;
                     at += __popc(who);
                 }
-                __syncwarp();
-#pragma unroll
-                for (int k = 0; k < kFew; ++k) v[k] = lane + 32 * k < at ? kept[lane + 32 * k] : -INFINITY;
-                above = n_upper;
-                is_few = true;
             }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < kFew; ++k) v[k] = lane + 32 * k < at ? kept[lane + 32 * k] : -INFINITY;
+            above = n_upper;
+            is_few = true;
         }
         T = __fdiv_rn(__fadd_rn(lower, upper), 2.0f);
         n = count(T);
@@ -554,12 +587,11 @@ int af_launch(AfParams p, int sup0, int sup1, int smooth0, int smooth1, int thr0
             af_ecc_kernel<<<(n + kEccFrames - 1) / kEccFrames, kEccFrames, ecc_smem(p.n_range), stream>>>(p);
         else
             af_ecc_long_kernel<<<(n + 127) / 128, 128, 0, stream>>>(p);
-        const int ctas = (n + 7) / 8;
-        if (p.n_range <= 8 * 32) af_threshold_kernel<8><<<ctas, 256, 0, stream>>>(p);
-        else if (p.n_range <= 20 * 32) af_threshold_kernel<20><<<ctas, 256, 0, stream>>>(p);
-        else if (p.n_range <= 40 * 32) af_threshold_kernel<40><<<ctas, 256, 0, stream>>>(p);
-        else if (p.n_range <= 80 * 32) af_threshold_kernel<80><<<ctas, 256, 0, stream>>>(p);
-        else af_threshold_kernel<0><<<ctas, 256, 0, stream>>>(p);
+        const int ctas = (n + kThrFrames - 1) / kThrFrames;
+        if (p.n_range > 32 * kFew && thr_smem(p.n_range) <= kThrSmem)
+            af_threshold_kernel<true><<<ctas, 32 * kThrFrames, thr_smem(p.n_range), stream>>>(p);
+        else
+            af_threshold_kernel<false><<<ctas, 32 * kThrFrames, 0, stream>>>(p);
         launches += 2;
     }
     if (out1 > out0) {
