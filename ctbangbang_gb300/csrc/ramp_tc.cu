@@ -210,24 +210,42 @@ __device__ __forceinline__ void row_exponents(float m, float sum_abs_taps, int *
 // Scales of a row: scale = 2^e_out (what the backprojector multiplies by) and
 // the epilogue's factor 2^(e_in - 10 - e_out) from the accumulator to the
 // stored value.
-__device__ __forceinline__ void write_row(const float *__restrict__ xr, int n, int lane, int e_in, int e_out,
-                                          __half *__restrict__ hr, __half *__restrict__ lr, float *scale,
-                                          float *mult)
+__device__ __forceinline__ void write_scales(int e_in, int e_out, float *scale, float *mult)
 {
-    if (lane == 0) {
-        *scale = ldexpf(1.0f, e_out);
-        *mult = ldexpf(1.0f, e_in - kTapExp - e_out);
-    }
-    const float s = ldexpf(1.0f, -e_in);
-    for (int i = lane; i < n; i += 32) {
-        float v = xr[i] * s;  // exact: a power of two
-        __half h = __float2half_rn(v);
-        hr[i] = h;
-        lr[i] = __float2half_rn(v - __half2float(h));
-    }
+    *scale = ldexpf(1.0f, e_out);
+    *mult = ldexpf(1.0f, e_in - kTapExp - e_out);
 }
 
-// One warp per row: max |x|, its exponents, then x_hi, x_lo.
+// Four consecutive samples (VEC: one 16-byte load)
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float *x)
+{
+    if constexpr (VEC) return *reinterpret_cast<const float4 *>(x);
+    return make_float4(x[0], x[1], x[2], x[3]);
+}
+
+__device__ __forceinline__ float max4(float m, float4 v)
+{
+    return fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+}
+
+// Four samples times s (a power of two: exact) as FP16 hi + lo.
+__device__ __forceinline__ void store4(float4 x, float s, __half *hi, __half *lo)
+{
+    const float v[4] = {x.x * s, x.y * s, x.z * s, x.w * s};
+    __half h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        h[i] = __float2half_rn(v[i]);
+        l[i] = __float2half_rn(v[i] - __half2float(h[i]));
+    }
+    *reinterpret_cast<uint2 *>(hi) = *reinterpret_cast<const uint2 *>(h);
+    *reinterpret_cast<uint2 *>(lo) = *reinterpret_cast<const uint2 *>(l);
+}
+
+// One warp per row: max |x|, its exponents, then x_hi, x_lo.  The row (at most
+// 1536 samples, a multiple of 64) is read once, into registers.
+template <bool VEC>
 __global__ void __launch_bounds__(256) ramp_tc_split_kernel(const float *__restrict__ x, size_t n_lines, int n,
                                                             float sum_abs_taps, __half *__restrict__ hi,
                                                             __half *__restrict__ lo, float *__restrict__ scale,
@@ -238,42 +256,81 @@ __global__ void __launch_bounds__(256) ramp_tc_split_kernel(const float *__restr
     const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
     for (size_t row = warp; row < n_lines; row += warps) {
         const float *xr = x + row * (size_t)n;
+        float4 v[kNPad / 128];
         float m = 0.0f;
-        for (int i = lane; i < n; i += 32) m = fmaxf(m, fabsf(xr[i]));
+#pragma unroll
+        for (int k = 0; k < kNPad / 128; ++k)
+            if (4 * (lane + 32 * k) < n) v[k] = load4<VEC>(xr + 4 * (lane + 32 * k));
+#pragma unroll
+        for (int k = 0; k < kNPad / 128; ++k)
+            if (4 * (lane + 32 * k) < n) m = max4(m, v[k]);
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
         int e_in, e_out;
         row_exponents(m, sum_abs_taps, &e_in, &e_out);
-        write_row(xr, n, lane, e_in, e_out, hi + row * (size_t)n, lo + row * (size_t)n, scale + row, mult + row);
+        if (lane == 0) write_scales(e_in, e_out, scale + row, mult + row);
+        const float s = ldexpf(1.0f, -e_in);
+#pragma unroll
+        for (int k = 0; k < kNPad / 128; ++k) {
+            const int i = 4 * (lane + 32 * k);
+            if (i < n) store4(v[k], s, hi + row * (size_t)n + i, lo + row * (size_t)n + i);
+        }
     }
 }
 
-// The same split with one exponent per view: a CTA per view of rpv rows (8
-// warps), the exponent from the largest |x| of all its rows.
-__global__ void __launch_bounds__(256) ramp_tc_split_view_kernel(const float *__restrict__ x, size_t n_lines, int n,
-                                                                 int rpv, float sum_abs_taps, __half *__restrict__ hi,
-                                                                 __half *__restrict__ lo, float *__restrict__ scale,
-                                                                 float *__restrict__ mult)
+// The same split with one exponent per view: a CTA per view of rpv rows, the
+// exponent from the largest |x| of all its rows.  The view is read twice, so
+// few CTAs an SM, each with many 16-byte loads in flight, leave the second
+// reading to L2 (64 rows of 1472 are 377 KB; eight CTAs of scalar loads ran
+// through HBM twice).  With the row form: 82 176 rows in views of 64 take
+// 1152 us with the filter instead of 1220, 12 800 rows of 1024 103 instead of
+// 111; two or four CTAs an SM the same.
+constexpr int kSplitThreads = 512, kSplitCtas = 3;
+
+template <bool VEC>
+__global__ void __launch_bounds__(kSplitThreads, kSplitCtas)
+    ramp_tc_split_view_kernel(const float *__restrict__ x, size_t n_lines, int n, int rpv, float sum_abs_taps,
+                              __half *__restrict__ hi, __half *__restrict__ lo, float *__restrict__ scale,
+                              float *__restrict__ mult)
 {
-    __shared__ float red[8];
+    __shared__ float red[kSplitThreads / 32];
+    constexpr int kUnroll = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (size_t g0 = (size_t)blockIdx.x * rpv; g0 < n_lines; g0 += (size_t)gridDim.x * rpv) {
-        const size_t g1 = g0 + rpv < n_lines ? g0 + rpv : n_lines;
-        float m = 0.0f;
-        for (size_t row = g0 + warp; row < g1; row += 8) {
-            const float *xr = x + row * (size_t)n;
-            for (int i = lane; i < n; i += 32) m = fmaxf(m, fabsf(xr[i]));
+    const size_t g0 = (size_t)blockIdx.x * rpv;
+    const int rows = (int)(g0 + rpv < n_lines ? rpv : n_lines - g0), n4 = rows * (n / 4);
+    const float *src = x + g0 * (size_t)n;
+    __half *h = hi + g0 * (size_t)n, *l = lo + g0 * (size_t)n;
+    float m = 0.0f;
+    for (int i0 = threadIdx.x; i0 < n4; i0 += kUnroll * kSplitThreads) {
+        float4 v[kUnroll];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const int i = i0 + u * kSplitThreads;
+            v[u] = i < n4 ? load4<VEC>(src + 4 * (size_t)i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) red[warp] = m;
-        __syncthreads();
-        m = red[0];
-        for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w]);
-        __syncthreads();
-        int e_in, e_out;
-        row_exponents(m, sum_abs_taps, &e_in, &e_out);
-        for (size_t row = g0 + warp; row < g1; row += 8)
-            write_row(x + row * (size_t)n, n, lane, e_in, e_out, hi + row * (size_t)n, lo + row * (size_t)n,
-                      scale + row, mult + row);
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) m = max4(m, v[u]);
+    }
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) red[warp] = m;
+    __syncthreads();
+    m = red[0];
+    for (int w = 1; w < kSplitThreads / 32; ++w) m = fmaxf(m, red[w]);
+    int e_in, e_out;
+    row_exponents(m, sum_abs_taps, &e_in, &e_out);
+    for (int r = threadIdx.x; r < rows; r += kSplitThreads) write_scales(e_in, e_out, scale + g0 + r, mult + g0 + r);
+    const float s = ldexpf(1.0f, -e_in);
+    for (int i0 = threadIdx.x; i0 < n4; i0 += kUnroll * kSplitThreads) {
+        float4 v[kUnroll];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const int i = i0 + u * kSplitThreads;
+            if (i < n4) v[u] = load4<VEC>(src + 4 * (size_t)i);
+        }
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const int i = i0 + u * kSplitThreads;
+            if (i < n4) store4(v[u], s, h + 4 * (size_t)i, l + 4 * (size_t)i);
+        }
     }
 }
 
@@ -652,14 +709,16 @@ int launch_ramp_tc(const RampTcPlan &plan, const float *d_rows, size_t n_lines, 
         set_error("ramp filter (tensor cores): %d rows per view do not divide %d", rows_per_view, BM);
         return CTBB_ERR_ARGUMENT;
     }
+    const bool vec = reinterpret_cast<uintptr_t>(d_rows) % 16 == 0;
     if (rows_per_view > 0) {
-        int blocks = (int)std::min<size_t>((n_lines + rows_per_view - 1) / rows_per_view, (size_t)num_sms() * 8);
-        ramp_tc_split_view_kernel<<<blocks, 256, 0, stream>>>(d_rows, n_lines, n, rows_per_view, plan.sum_abs_taps,
-                                                              xh, xl, d_scale, mult);
+        const unsigned views = (unsigned)((n_lines + rows_per_view - 1) / rows_per_view);
+        auto *split = vec ? ramp_tc_split_view_kernel<true> : ramp_tc_split_view_kernel<false>;
+        split<<<views, kSplitThreads, 0, stream>>>(d_rows, n_lines, n, rows_per_view, plan.sum_abs_taps, xh, xl,
+                                                   d_scale, mult);
     } else {
         int blocks = (int)std::min<size_t>((n_lines + 7) / 8, (size_t)num_sms() * 16);
-        ramp_tc_split_kernel<<<blocks, 256, 0, stream>>>(d_rows, n_lines, n, plan.sum_abs_taps, xh, xl, d_scale,
-                                                         mult);
+        auto *split = vec ? ramp_tc_split_kernel<true> : ramp_tc_split_kernel<false>;
+        split<<<blocks, 256, 0, stream>>>(d_rows, n_lines, n, plan.sum_abs_taps, xh, xl, d_scale, mult);
     }
     count_launch();
     CTBB_CUDA_TRY(cudaGetLastError());
