@@ -879,6 +879,7 @@ int build_backproject_tables(const struct recon_metadata &mr, BackprojectTables 
     t->nht = d.n_half_turns;
     t->n_half = (int)(cg.n_proj_turn / 2);
     t->n_slices = (int)mr.ri.n_slices_block;
+    t->n_views = 0;
     t->views.resize((size_t)t->n_half * t->nht * 4);
     t->theta.resize((size_t)t->n_half * t->nht);
     for (int i = 0; i < t->n_half; ++i)
@@ -901,6 +902,7 @@ int build_backproject_tables(const struct recon_metadata &mr, BackprojectTables 
 
 void BackprojectTables::set_view_row(int i, int k, unsigned row)
 {
+    n_views = std::max(n_views, row + 1);
     uint32_t bits = row;
     std::memcpy(&views[((size_t)i * nht + k) * 4], &bits, sizeof(bits));
 }
@@ -932,12 +934,7 @@ int make_backproject_params(const struct recon_metadata &mr, const BackprojectTa
     p.n_rows = (int)cg.n_rows;
     p.nht = t.nht;
     p.n_half = t.n_half;
-    p.n_views = 0;
-    for (size_t v = 0; v < t.views.size(); v += 4) {
-        uint32_t row;
-        std::memcpy(&row, &t.views[v], sizeof(row));
-        p.n_views = std::max(p.n_views, (int)row + 1);
-    }
+    p.n_views = (int)t.n_views;
     p.pix_x = rp.recon_fov / (float)rp.nx;
     p.pix_y = rp.recon_fov / (float)rp.ny;
     p.x_c = (float)(rp.nx - 1) / 2.0f;

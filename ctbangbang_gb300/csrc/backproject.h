@@ -21,6 +21,7 @@ struct BackprojectTables {
     std::vector<float> views;
     std::vector<float> theta;  // [n_half][nht]: theta of view (i, k)
     std::vector<float> zpos;   // [n_slices]
+    unsigned n_views = 0;      // views the buffer holds: one past the last row index set
     void set_view_row(int i, int k, unsigned row);
 };
 
@@ -34,7 +35,6 @@ struct BpParams {
     const float *theta;    // [n_half][nht] theta (the last-turn border recheck)
     const float *zpos;     // [n_slices_block]
     int nx, ny, n_slices, nos, n_rows, nht, n_half;
-    int n_views;           // views the rows buffer holds (one past the last of the table's row indices)
     float pix_x, pix_y, x_c, y_c, x0, y0;  // x = pix_x * (xi - x_c) + x0
     float ds_half;         // r_f fai / 2
     float inv_ds_half;     // 1 / ds_half
@@ -56,6 +56,7 @@ struct BpParams {
     int col_zpt;           // column form: slices per thread (a multiple of 8, at most 32)
     int n_achunks;         // column form: angle chunks (grid z = slice chunks x angle chunks)
     float *partial;        // n_achunks > 1: [n_achunks][n_slices][ny][nx] unscaled image sums
+    int n_views;           // staged form: views the rows buffer holds (one past the last of the table's row indices)
 };
 
 // A launch shape: slices per thread, threads per CTA, CTAs per SM the kernel

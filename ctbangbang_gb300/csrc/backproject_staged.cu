@@ -46,6 +46,7 @@ namespace {
 constexpr int kGroups = 4;          // slice groups of 8: the block's 32 slices; visits of a step
 constexpr int kRecords = 192;       // visits of one segment of angles
 constexpr int kTileY = 8;           // voxel columns of a tile along y
+constexpr int kWideVisits = 608;    // staged_shape: most tiles x half turns of the 8 x 8 tile
 constexpr int kBoxRows = 8;         // detector rows of a TMA copy
 constexpr float kBoxMargin = 0.05f; // rows / channels added around the box's bounds
 // class of a visit for a slice group
@@ -627,6 +628,16 @@ bool staged_shape(const BpParams &p, StagedShape *out)
         const float wx = (float)(tile_x(c.cw) - 1) * std::fabs(p.pix_x), wy = (float)(kTileY - 1) * std::fabs(p.pix_y);
         const float span = (std::sqrt(wx * wx + wy * wy) + 4e-3f) * std::fabs(p.inv_ds_half) + 2.0f * kBoxMargin + 0.01f;
         if (!(span < 1000.0f)) continue;
+        // Coarse pixels (8 x 8 tiles, wide boxes) copy more per voxel than the
+        // column form gathers; their four warps per 32 columns pay where the
+        // column form has too few CTAs, or does not hold the window.  ms
+        // against the column form, by tiles x half turns: 93^2, 576: 0.47 /
+        // 0.78; 109^2, 588: 0.53 / 0.69; 133 x 99, 884: 0.35 / 0.30; 118^2,
+        // 1125: 0.83 / 0.80; 171^2, 2420: 1.89 / 1.66; 231 x 207, 3016: 3.63 /
+        // 3.29.
+        if (c.cw == 2 && p.nht <= kColumnMaxHalfTurns &&
+            ((p.nx + 7) / 8) * ((p.ny + kTileY - 1) / kTileY) * p.nht > kWideVisits)
+            continue;
         // channels from the first, moved down to a multiple of 4, to the one past the last
         if ((int)std::floor(span) + 3 + 3 > c.pitch) continue;
         // the whole of a view's rows fits a half, and at most four of them are
