@@ -279,9 +279,9 @@ __global__ void __launch_bounds__(256) ramp_tc_split_kernel(const float *__restr
 
 // The same split with one exponent per view: a CTA per view of rpv rows, the
 // exponent from the largest |x| of all its rows.  The view is read twice, so
-// few CTAs an SM, each with many 16-byte loads in flight, leave the second
-// reading to L2 (64 rows of 1472 are 377 KB; eight CTAs of scalar loads ran
-// through HBM twice).  With the row form: 82 176 rows in views of 64 take
+// few CTAs an SM, each with many 16-byte loads in flight, leave most of the
+// second reading to L2 (64 rows of 1472 are 377 KB; views of 128 rows still
+// come from HBM twice, at 6.9 TB/s).  With the row form: 82 176 rows in views of 64 take
 // 1152 us with the filter instead of 1220, 12 800 rows of 1024 103 instead of
 // 111; two or four CTAs an SM the same.
 constexpr int kSplitThreads = 512, kSplitCtas = 3;
