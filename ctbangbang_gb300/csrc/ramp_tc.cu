@@ -279,20 +279,22 @@ __global__ void __launch_bounds__(256) ramp_tc_split_kernel(const float *__restr
 
 // The same split with one exponent per view: a CTA per view of rpv rows, the
 // exponent from the largest |x| of all its rows.  The view is read twice, so
-// few CTAs an SM, each with many 16-byte loads in flight, leave most of the
-// second reading to L2 (64 rows of 1472 are 377 KB; views of 128 rows still
-// come from HBM twice, at 6.9 TB/s).  With the row form: 82 176 rows in views of 64 take
-// 1152 us with the filter instead of 1220, 12 800 rows of 1024 103 instead of
-// 111; two or four CTAs an SM the same.
-constexpr int kSplitThreads = 512, kSplitCtas = 3;
+// large ones take one CTA of 1024 threads an SM, each with many 16-byte loads
+// in flight, which leaves the second reading to L2 (64 rows of 1472 are 377 KB;
+// eight CTAs of scalar loads ran through HBM twice); small ones take CTAs of
+// 256 threads, as many as fit, since their chain of loads, maximum and stores is
+// short of work.  82 176 rows of 1472 in views of 64, with the filter: 1220 us
+// with scalar loads, 1113 so, 1162 with 256 threads; 51 200 rows of 512 in views
+// of 32: 227, 235 with 1024 threads; of 128 in views of 16: 76 and 110.
+constexpr int kSplitLarge = 32768;  // samples of a view from which it takes 1024 threads
 
-template <bool VEC>
-__global__ void __launch_bounds__(kSplitThreads, kSplitCtas)
+template <bool VEC, int THREADS>
+__global__ void __launch_bounds__(THREADS)
     ramp_tc_split_view_kernel(const float *__restrict__ x, size_t n_lines, int n, int rpv, float sum_abs_taps,
                               __half *__restrict__ hi, __half *__restrict__ lo, float *__restrict__ scale,
                               float *__restrict__ mult)
 {
-    __shared__ float red[kSplitThreads / 32];
+    __shared__ float red[THREADS / 32];
     constexpr int kUnroll = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const size_t g0 = (size_t)blockIdx.x * rpv;
@@ -300,11 +302,11 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitCtas)
     const float *src = x + g0 * (size_t)n;
     __half *h = hi + g0 * (size_t)n, *l = lo + g0 * (size_t)n;
     float m = 0.0f;
-    for (int i0 = threadIdx.x; i0 < n4; i0 += kUnroll * kSplitThreads) {
+    for (int i0 = threadIdx.x; i0 < n4; i0 += kUnroll * THREADS) {
         float4 v[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            const int i = i0 + u * kSplitThreads;
+            const int i = i0 + u * THREADS;
             v[u] = i < n4 ? load4<VEC>(src + 4 * (size_t)i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
 #pragma unroll
@@ -314,21 +316,21 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitCtas)
     if (lane == 0) red[warp] = m;
     __syncthreads();
     m = red[0];
-    for (int w = 1; w < kSplitThreads / 32; ++w) m = fmaxf(m, red[w]);
+    for (int w = 1; w < THREADS / 32; ++w) m = fmaxf(m, red[w]);
     int e_in, e_out;
     row_exponents(m, sum_abs_taps, &e_in, &e_out);
-    for (int r = threadIdx.x; r < rows; r += kSplitThreads) write_scales(e_in, e_out, scale + g0 + r, mult + g0 + r);
+    for (int r = threadIdx.x; r < rows; r += THREADS) write_scales(e_in, e_out, scale + g0 + r, mult + g0 + r);
     const float s = ldexpf(1.0f, -e_in);
-    for (int i0 = threadIdx.x; i0 < n4; i0 += kUnroll * kSplitThreads) {
+    for (int i0 = threadIdx.x; i0 < n4; i0 += kUnroll * THREADS) {
         float4 v[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            const int i = i0 + u * kSplitThreads;
+            const int i = i0 + u * THREADS;
             if (i < n4) v[u] = load4<VEC>(src + 4 * (size_t)i);
         }
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            const int i = i0 + u * kSplitThreads;
+            const int i = i0 + u * THREADS;
             if (i < n4) store4(v[u], s, h + 4 * (size_t)i, l + 4 * (size_t)i);
         }
     }
@@ -712,8 +714,10 @@ int launch_ramp_tc(const RampTcPlan &plan, const float *d_rows, size_t n_lines, 
     const bool vec = reinterpret_cast<uintptr_t>(d_rows) % 16 == 0;
     if (rows_per_view > 0) {
         const unsigned views = (unsigned)((n_lines + rows_per_view - 1) / rows_per_view);
-        auto *split = vec ? ramp_tc_split_view_kernel<true> : ramp_tc_split_view_kernel<false>;
-        split<<<views, kSplitThreads, 0, stream>>>(d_rows, n_lines, n, rows_per_view, plan.sum_abs_taps, xh, xl,
+        const bool large = (size_t)rows_per_view * n >= kSplitLarge;
+        auto *split = vec ? (large ? ramp_tc_split_view_kernel<true, 1024> : ramp_tc_split_view_kernel<true, 256>)
+                          : (large ? ramp_tc_split_view_kernel<false, 1024> : ramp_tc_split_view_kernel<false, 256>);
+        split<<<views, large ? 1024 : 256, 0, stream>>>(d_rows, n_lines, n, rows_per_view, plan.sum_abs_taps, xh, xl,
                                                    d_scale, mult);
     } else {
         int blocks = (int)std::min<size_t>((n_lines + 7) / 8, (size_t)num_sms() * 16);
