@@ -104,7 +104,7 @@ void axis_taps(float idx, int dim, int *i0, int *i1, float *u, float *one_minus_
     float fl = std::floor(idx);
     *u = idx - fl;
     *one_minus_u = 1.0f - *u;
-    *i0 = (int)fl;
+    *i0 = fl == fl ? (int)fl : 0;  // a channel past 90 degrees: weights that are not numbers, taps in range
     *i1 = (idx == (float)dim - 1.0f) ? *i0 : *i0 + 1;
 }
 
@@ -254,6 +254,10 @@ int build_rebin_tables(const struct recon_metadata &mr, RebinTables *t)
             auto reads = [&](int ch, int e, float t_alpha) {
                 lo = std::min(lo, ch);
                 hi = std::max(hi, ch);
+                if (!std::isfinite(t_alpha + t->focal_offset[two_stage ? 2 * s + e : s])) {  // no box holds its views (see staged_frames)
+                    tile.t_min[e] = -INFINITY;
+                    tile.t_max[e] = INFINITY;
+                }
                 tile.t_min[e] = std::min(tile.t_min[e], t_alpha);
                 tile.t_max[e] = std::max(tile.t_max[e], t_alpha);
             };
@@ -486,7 +490,6 @@ __global__ void rebin_two_stage_kernel(RebinParams p)
 // us on a config-2 window where 64 (37 KB, 6 CTAs) move 2.55 GB and take 415;
 // 32 views to a box 550, 256 threads 454; gathering 611.  What bounds it now
 // is the L2 traffic of the boxes (6.1 TB/s) beside 4.9 TB/s of HBM.
-constexpr int kStagedViews = 16;
 constexpr int kNarrowBox = 40, kWideBox = 48;  // channels of a box: a tile's, wider with a z flying focal spot
 
 struct StagedRebin {
@@ -507,15 +510,11 @@ __global__ void __launch_bounds__(128) rebin_staged_kernel(RebinParams p, Staged
     const int v0 = p.v_begin + blockIdx.z * kStagedViews, v1 = min(v0 + kStagedViews, p.v_end);
     const RebinTile tile = g.tiles[side * g.n_tiles + blockIdx.x];
     const int q0 = TWO ? 2 * side : side;  // the side's first focal spot
-    // first frame of each box: one before the lowest view coordinate (its
-    // float rounding is far below a frame), inside the scan as the taps are
-    int f0[kSpots];
+    int f0[kSpots];  // first frame of each box
 #pragma unroll
     for (int e = 0; e < kSpots; ++e) {
         const float off = p.n_ffs == 1 ? 0.0f : p.focal_offset[q0 + e];
-        const float c = tile.t_max[e] + off + (float)(q0 + e);
-        const int lowest = (v0 + p.add) - (int)ceilf(c / (float)p.n_ffs) - 1;
-        f0[e] = min(max(lowest, 0), p.n_proj - 1);
+        f0[e] = rebin_box_first(tile.t_max[e], off, q0 + e, p.n_ffs, v0 + p.add, p.n_proj);
     }
     const uint32_t bar = smem_address(&full);
     if (threadIdx.x == 0) {
@@ -605,9 +604,6 @@ __global__ void __launch_bounds__(128) rebin_staged_kernel(RebinParams p, Staged
     }
 }
 
-// Frames of the staged form's boxes, or 0 where it does not apply: rows off
-// 16-byte boundaries, a tile wider than the box, or t_alpha moving so fast
-// that two boxes do not fit beside another CTA's (few, wide channels).
 int staged_frames(const RebinTables &t, const float *d_raw, int spots, int *channels)
 {
     if (t.n_channels % 4 != 0 || ((uintptr_t)d_raw & 15) != 0) return 0;

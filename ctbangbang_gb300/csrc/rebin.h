@@ -55,6 +55,25 @@ struct DeviceRebinTables {
 };
 
 int build_rebin_tables(const struct recon_metadata &mr, RebinTables *t);
+
+// The staged kernel (rebin.cu): a CTA's views of one side, and the first frame
+// of its box of focal spot q (offset off, largest t_alpha t_max): one before
+// the lowest view coordinate (whose float rounding is far below a frame),
+// inside the scan as the taps are.
+constexpr int kStagedViews = 16;
+__host__ __device__ inline int rebin_box_first(float t_max, float off, int q, int n_ffs, int proj, int n_proj)
+{
+    const float c = t_max + off + (float)q;
+    const int lowest = proj - (int)ceilf(c / (float)n_ffs) - 1;
+    return lowest < 0 ? 0 : (lowest > n_proj - 1 ? n_proj - 1 : lowest);
+}
+// Frames of the staged kernel's boxes, or 0 where it does not apply: rows off
+// 16-byte boundaries, a tile wider than the box, t_alpha moving so fast that
+// two boxes do not fit beside another CTA's (few, wide channels), or a channel
+// whose t_alpha is not finite (past 90 degrees): the gathering kernel clamps
+// its view to the scan, but no box can be placed around it.
+int staged_frames(const RebinTables &t, const float *d_raw, int spots, int *channels);
+
 int upload_rebin_tables(const RebinTables &t, DeviceRebinTables *dt, cudaStream_t stream);
 // Views [v_begin, v_end) of the output (v_end < 0: all views).
 int launch_rebin(const RebinTables &t, const DeviceRebinTables &dt, const float *d_raw,
