@@ -55,3 +55,46 @@ def test_rebin_taps_lie_in_their_box(rebin_check, tmp_path, z, phi, channels, vi
                       n_slices=4)
     frames, outside = _rebin(rebin_check, spec, tmp_path)
     assert (frames > 0) == staged and outside == 0, (frames, outside)
+
+
+@pytest.fixture(scope="module")
+def box_check(lib):
+    return _native("staged_backproject")
+
+
+def _boxes(check, spec, tmp_path, n_slices=None, angle_step=1):
+    mr = scans.plan_spec(spec, str(tmp_path))
+    L.call("ctbb_update_block_info", C.byref(mr))
+    if n_slices is not None:
+        mr.ri.n_slices_block = n_slices
+    visits, outside, misread = C.c_longlong(-1), C.c_longlong(-1), C.c_longlong(-1)
+    assert check.check_staged_boxes(C.byref(mr), angle_step, C.byref(visits), C.byref(outside), C.byref(misread)) == 0
+    scans.free_plan(mr)
+    return visits.value, outside.value, misread.value
+
+
+# z, phi, raw rows, views per turn, channels, nx, ny, pitch, table
+BOXES = [(0, 0, 8, 96, 64, 17, 9, 1.0, "out"), (1, 1, 64, 192, 64, 33, 31, 0.8, "out"),
+         (0, 1, 32, 192, 96, 48, 24, 1.4, "in"), (1, 0, 10, 101, 64, 40, 24, 0.6, "out")]
+
+
+@pytest.mark.parametrize("z,phi,rows,views,channels,nx,ny,pitch,table", BOXES)
+def test_backprojection_samples_lie_in_their_box(box_check, tmp_path, z, phi, rows, views, channels, nx, ny, pitch,
+                                                 table):
+    spec = scans.tiny(z, phi, n_rows_raw=rows, n_proj_turn=views, n_channels=channels, nx=nx, ny=ny, n_slices=6,
+                      pitch=pitch, table_dir=table)
+    visits, outside, misread = _boxes(box_check, spec, tmp_path)
+    assert visits > 0 and outside == 0 and misread == 0, (visits, outside, misread)
+
+
+@pytest.mark.parametrize("n_slices", [1, 5, 9, 31])
+@pytest.mark.parametrize("z,phi,rows,channels,nx,ny,coll", [(0, 1, 64, 166, 35, 28, 0.3), (1, 0, 8, 60, 12, 14, 3.0),
+                                                            (1, 1, 16, 48, 33, 9, 1.0)])
+def test_slices_past_the_end_of_a_block(box_check, tmp_path, z, phi, rows, channels, nx, ny, coll, n_slices):
+    """A block of fewer slices than whole groups of 8: a warp reads for all 8."""
+    spec = scans.tiny(z, phi, n_rows_raw=rows, n_proj_turn=40, n_channels=channels, nx=nx, ny=ny, n_slices=4)
+    spec.coll = spec.slice_thickness = coll
+    spec.start_pos = scans.allowed_margin(spec) + 2.0
+    spec.turns = scans.needed_turns(spec)
+    visits, outside, misread = _boxes(box_check, spec, tmp_path, n_slices)
+    assert visits > 0 and outside == 0 and misread == 0, (visits, outside, misread)
