@@ -562,6 +562,14 @@ bool staged_shape(const BpParams &p, StagedShape *out)
         const float wx = (float)(tile_x(c.cw) - 1) * std::fabs(p.pix_x), wy = (float)(kTileY - 1) * std::fabs(p.pix_y);
         const float span = (std::sqrt(wx * wx + wy * wy) + 4e-3f) * std::fabs(p.inv_ds_half) + 2.0f * kBoxMargin + 0.01f;
         if (!(span < 1000.0f)) continue;
+        // visit_box bounds p and the ray position of a tile separately: the
+        // rectangle they span around the tile has to lie inside the source's
+        // circle too, or its distances to the source turn negative
+        // (tiles of tens of centimetres, on detectors of few channels)
+        const float hx = 0.5f * (float)(std::min(tile_x(c.cw), p.nx) - 1) * std::fabs(p.pix_x);
+        const float hy = 0.5f * (float)(std::min(kTileY, p.ny) - 1) * std::fabs(p.pix_y);
+        const float tx = rx - hx, ty = ry - hy;  // the outermost tile's centre
+        if (!(std::sqrt(tx * tx + ty * ty) + hx + hy < 0.95f * p.rf)) continue;
         // Coarse pixels (8 x 8 tiles, wide boxes) copy more per voxel than the
         // column form gathers; their four warps per 32 columns pay where the
         // column form has too few CTAs, or does not hold the window.  ms

@@ -98,3 +98,19 @@ def test_slices_past_the_end_of_a_block(box_check, tmp_path, z, phi, rows, chann
     spec.turns = scans.needed_turns(spec)
     visits, outside, misread = _boxes(box_check, spec, tmp_path, n_slices)
     assert visits > 0 and outside == 0 and misread == 0, (visits, outside, misread)
+
+
+# channels, nx, ny, field of view, origin
+COARSE = [(16, 19, 9, 374.0, 0.0), (16, 6, 6, 370.0, 0.0), (20, 12, 5, 300.0, 60.0), (24, 30, 30, 380.0, 0.0)]
+
+
+@pytest.mark.parametrize("channels,nx,ny,fov,x0", COARSE)
+@pytest.mark.parametrize("fan", [0.46, 1.2])
+def test_tiles_of_tens_of_centimetres(box_check, tmp_path, channels, nx, ny, fov, x0, fan):
+    """Few channels, large pixels: a tile's bounds may reach the source's circle
+    where its voxels do not; such images take another form."""
+    spec = scans.tiny(1, 1, n_rows_raw=32, n_proj_turn=100, n_channels=channels, nx=nx, ny=ny, n_slices=4,
+                      fan_angle_increment=fan / channels)
+    spec.recon_fov, spec.x_origin = fov, x0
+    visits, outside, misread = _boxes(box_check, spec, tmp_path)
+    assert outside == 0 and misread == 0, (visits, outside, misread)
