@@ -130,21 +130,30 @@ __global__ void __launch_bounds__(256, 4) af_copy_kernel(AfParams p)
     }
 }
 
+// STAGED: the CTA's windows, weighted, in shared memory (kSmoothSmem); an
+// averaging window past that (more than 12 161 frames) is read as it lies.  The sum
+// keeps the reference's order in both.
+constexpr size_t kSmoothSmem = 48 * 1024;
+
+__host__ __device__ constexpr size_t smooth_smem(int n_avg) { return (size_t)(127 + (size_t)n_avg) * sizeof(float); }
+
+template <bool STAGED>
 __global__ void af_smooth_kernel(AfParams p)
 {
-    // the CTA's windows, weighted, in shared memory; the sum keeps the
-    // reference's order
     extern __shared__ float win[];
     const int first = p.f0 + blockIdx.x * blockDim.x, n = min((int)blockDim.x, p.f1 - first);
     const float w = __fdiv_rn(1.0f, (float)p.n_avg);
     const int max_idx = p.P - 1;
-    for (int i = threadIdx.x; i < n + p.n_avg - 1; i += blockDim.x)
-        win[i] = __fmul_rn(w, p.sup[min(max(first - p.avg_offset + i, 0), max_idx)]);
-    __syncthreads();
+    auto weighted = [&](int i) { return __fmul_rn(w, p.sup[min(max(first - p.avg_offset + i, 0), max_idx)]); };
+    if (STAGED) {
+        for (int i = threadIdx.x; i < n + p.n_avg - 1; i += blockDim.x) win[i] = weighted(i);
+        __syncthreads();
+    }
     if ((int)threadIdx.x >= n) return;
     float acc = 0.0f;
 #pragma unroll 8
-    for (int i = 0; i < p.n_avg; i++) acc = __fadd_rn(acc, win[threadIdx.x + i]);
+    for (int i = 0; i < p.n_avg; i++)
+        acc = __fadd_rn(acc, STAGED ? win[threadIdx.x + i] : weighted((int)threadIdx.x + i));
     p.smooth[first + threadIdx.x] = acc;
 }
 
@@ -576,7 +585,11 @@ int af_launch(AfParams p, int sup0, int sup1, int smooth0, int smooth1, int thr0
     if (smooth1 > smooth0) {
         p.f0 = smooth0;
         p.f1 = smooth1;
-        af_smooth_kernel<<<(smooth1 - smooth0 + 127) / 128, 128, (size_t)(127 + p.n_avg) * sizeof(float), stream>>>(p);
+        const int ctas = (smooth1 - smooth0 + 127) / 128;
+        if (smooth_smem(p.n_avg) <= kSmoothSmem)
+            af_smooth_kernel<true><<<ctas, 128, smooth_smem(p.n_avg), stream>>>(p);
+        else
+            af_smooth_kernel<false><<<ctas, 128, 0, stream>>>(p);
         ++launches;
     }
     if (thr1 > thr0) {
