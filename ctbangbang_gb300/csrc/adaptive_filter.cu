@@ -58,6 +58,7 @@ struct AfParams {
     int n_range, range_offset;
     float strength;
     int f0, f1;  // frames this launch writes: [f0, f1) of the window [0, P)
+    int parts;   // af_filter_kernel: parts of a frame
 };
 
 // Groups of four consecutive samples of a frame; VEC: 16-byte accesses (whole
@@ -413,41 +414,135 @@ __device__ __forceinline__ void smooth_samples(const AfParams &p, const int2 *li
     }
 }
 
+// The same for a part of a frame, rows [row0, row1), that is dense in samples
+// above the threshold: tiles of kTileRows x kTileCols outputs with their halo
+// in shared memory, a thread for four consecutive channels of a row, so that a
+// tap fetched serves up to four sums (50 reads of shared memory per sample
+// instead of 125).  Column c of a tile row lies at (c mod 4, c / 4): lanes four
+// channels apart read consecutive words.  Every thread of the CTA calls it;
+// true if about a sixteenth of the part or more was above.
+constexpr int kTileRows = 4, kTileCols = 256;  // a warp per half row
+constexpr int kPlane = 68;  // (kTileCols + 4) / 4 words, rounded up against store conflicts
+constexpr int kTileRow = 4 * kPlane, kTileFrame = (kTileRows + 4) * kTileRow, kTileFloats = 5 * kTileFrame;
+
+__device__ __forceinline__ bool smooth_part(const AfParams &p, int f, float T, int row0, int row1, float *tile)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t frame = (size_t)p.R * p.N;
+    bool any = false, held = false;
+    for (int r0 = row0; r0 < row1; r0 += kTileRows)
+        for (int c0 = 0; c0 < p.N; c0 += kTileCols) {
+            const int n_rows = min(kTileRows, row1 - r0) + 4;
+            __syncthreads();  // the last tile is read
+            for (int q = warp; q < 5 * n_rows; q += 8) {
+                const int k = q / n_rows, tr = q - k * n_rows, gf = f + k - 2, gr = r0 + tr - 2;
+                const bool in = gf >= 0 && gf < p.P && gr >= 0 && gr < p.R;
+                const float *src = p.raw + (in ? (size_t)gf * frame + (size_t)gr * p.N : 0);
+                float *dst = tile + k * kTileFrame + tr * kTileRow + (lane & 3) * kPlane + (lane >> 2);
+                float x[(kTileCols + 4 + 31) / 32];
+#pragma unroll
+                for (int m = 0; m < (kTileCols + 4 + 31) / 32; ++m) {
+                    const int gc = c0 + lane + 32 * m - 2;
+                    x[m] = in && lane + 32 * m < kTileCols + 4 && gc >= 0 && gc < p.N ? __ldg(src + gc) : 0.0f;
+                }
+#pragma unroll
+                for (int m = 0; m < (kTileCols + 4 + 31) / 32; ++m)
+                    if (lane + 32 * m < kTileCols + 4) dst[8 * m] = x[m];
+            }
+            __syncthreads();
+            const int tr = warp & 3, tc = 32 * (warp >> 2) + lane, gr = r0 + tr, gc = c0 + 4 * tc;
+            if (gr >= row1 || gc >= p.N) continue;
+            const float *at = tile + tr * kTileRow + tc;
+            float x[4], val[4] = {};
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {  // channel gc + t - 2
+                float v[25];
+#pragma unroll
+                for (int m = 0; m < 25; ++m)
+                    v[m] = at[(m % 5) * kTileFrame + (m / 5) * kTileRow + (t & 3) * kPlane + (t >> 2)];
+                if (t >= 2 && t < 6) x[t - 2] = v[12];
+#pragma unroll
+                for (int o = 0; o < 4; ++o)
+                    if (t - o >= 0 && t - o < 5) {
+#pragma unroll
+                        for (int m = 0; m < 25; ++m)
+                            val[o] = __fadd_rn(val[o], __fmul_rn(v[m], (float)(tri1(t - o) + tri1(m / 5) + tri1(m % 5) + 1)));
+                    }
+            }
+            held = true;
+            int nj = 0, nk = 0, sj = 0, sk = 0;
+#pragma unroll
+            for (int d = 0; d < 5; ++d) {
+                if (gr + d - 2 >= 0 && gr + d - 2 < p.R) { nj++; sj += tri1(d); }
+                if (f + d - 2 >= 0 && f + d - 2 < p.P) { nk++; sk += tri1(d); }
+            }
+#pragma unroll
+            for (int o = 0; o < 4; ++o) {
+                const int c = gc + o;
+                if (c >= p.N || !(x[o] > T)) continue;
+                any = true;
+                int ni = 0, si = 0;
+#pragma unroll
+                for (int d = 0; d < 5; ++d)
+                    if (c + d - 2 >= 0 && c + d - 2 < p.N) { ni++; si += tri1(d); }
+                const float norm = (float)(nj * nk * si + ni * nk * sj + ni * nj * sk + ni * nj * nk);
+                p.out[(size_t)f * frame + (size_t)gr * p.N + c] = __fmul_rn(__fdiv_rn(1.0f, norm), val[o]);
+            }
+        }
+    // half of the threads with a sample of theirs above, at a dozen samples each
+    return 2 * __syncthreads_count(any) >= __syncthreads_count(held);
+}
+
 // Step 5, on a copy of the frames (af_copy_kernel): only frames whose maximum
 // exceeds their threshold are read again (thresholds lie between means of
 // maxima, so they are never negative), one in twenty at strength 1.  They come
-// in short runs, so a frame is cut into kParts parts, and each CTA serves one
-// part of every `lanes`-th frame: it lists the samples above the threshold in
-// shared memory, over all its frames, and smooths them together, or earlier
+// in short runs, so a frame is cut into up to kParts parts, and each CTA serves
+// one part of every `lanes`-th frame: it lists the samples above the threshold
+// in shared memory, over all its frames, and smooths them together, or earlier
 // when the list runs full.  Bound by the waits of its chain (thresholds, four
 // rounds of loads at a time, taps): 42 us for the window above, where a CTA per
 // frame with a thread per listed sample took 69 us; 4 or 16 parts take 2 %
 // longer for the call, 8 rounds at a time 4 %.
+// A warp smooths four listed samples at a time, which a part with many leaves
+// to smooth_part: when the list fills up and a sixteenth of the part at hand
+// is in it, that part and those after it are smoothed as tiles, until one is
+// not dense (a listed sample costs some sixteen times a tile's).  2816 frames
+// of 736 x 32 with 90 % of the samples above: 15.3 ms all from the list, 1.44
+// so; of 738 x 32 14.7 and 1.44 (1.53 when every sample went through a tile);
+// with 3 % above 0.78 and 0.51.
 constexpr int kParts = 8;
 constexpr int kAhead = 4;
-constexpr int kListRoom = 4 * 256;  // samples a round can add
+constexpr int kListRoom = 4 * 256;  // samples a round can add, and the fewest of a part
 constexpr int kSmoothListMax = 2 * kListRoom;
 constexpr int kFilterCtas = 2;
 
 template <bool VEC>
 __global__ void __launch_bounds__(256, kFilterCtas) af_filter_kernel(AfParams p)
 {
-    __shared__ int2 list[kSmoothListMax];
-    __shared__ float taps[8][125 * kWarpSamples];
+    // the list and the warps' taps, or a tile
+    constexpr int kTaps = 125 * kWarpSamples;
+    static_assert(2 * kSmoothListMax + 8 * kTaps <= kTileFloats, "the list and the taps lie in the tile's place");
+    __shared__ __align__(16) float work[kTileFloats];
+    int2 *list = reinterpret_cast<int2 *>(work);
+    float *taps = work + 2 * kSmoothListMax + threadIdx.x / 32 * kTaps;
     __shared__ int active[256];
     __shared__ float active_thr[256];
-    __shared__ int n_list, n_active;
-    const int part = blockIdx.x % kParts, lanes = gridDim.x / kParts;
+    __shared__ int n_list, n_active, part_at;
+    const int part = blockIdx.x % p.parts, lanes = gridDim.x / p.parts;
     const size_t frame = (size_t)p.R * p.N;
     const int n_frame = (int)frame, n4 = (n_frame + 3) / 4;
-    const int g0 = (int)((long long)part * n4 / kParts), g1 = (int)((long long)(part + 1) * n4 / kParts);
-    auto smooth_listed = [&] {
-        const int n = n_list;
+    // a part is a number of rows, all but the last part's a multiple of 4 (whole
+    // groups, and whole tiles)
+    const int rows4 = (p.R + 3) / 4, row0 = 4 * (part * rows4 / p.parts);
+    const int row1 = min(4 * ((part + 1) * rows4 / p.parts), p.R);
+    const int g0 = row0 / 4 * p.N, g1 = row1 < p.R ? row1 / 4 * p.N : n4;
+    auto smooth_listed = [&](int n) {
         for (int j = (int)threadIdx.x / 32 * kWarpSamples; j < n; j += 8 * kWarpSamples)
-            smooth_samples(p, list + j, n - j, taps[threadIdx.x / 32]);
+            smooth_samples(p, list + j, n - j, taps);
     };
+    bool dense = false;  // the last part was; the list is empty
     if (threadIdx.x == 0) n_list = 0;
-    for (int first = p.f0 + (int)blockIdx.x / kParts; first < p.f1; first += 256 * lanes) {
+    for (int first = p.f0 + (int)blockIdx.x / p.parts; first < p.f1; first += 256 * lanes) {
         if (threadIdx.x == 0) n_active = 0;
         __syncthreads();
         const int f = first + (int)threadIdx.x * lanes;
@@ -461,7 +556,14 @@ __global__ void __launch_bounds__(256, kFilterCtas) af_filter_kernel(AfParams p)
         const int n = n_active;
         // rounds of 256 groups, the loads of kAhead of them in flight
         const int rounds = (g1 - g0 + 255) / 256;
-        for (int w0 = 0; w0 < n * rounds; w0 += kAhead) {
+        for (int w0 = 0, w1; w0 < n * rounds; w0 = w1) {
+            if (dense) {  // w0 is the first round of a part
+                const int a = w0 / rounds;
+                dense = smooth_part(p, active[a], active_thr[a], row0, row1, work);
+                w1 = w0 + rounds;
+                continue;
+            }
+            w1 = w0 + kAhead;
             float4 v[kAhead];
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {
@@ -471,7 +573,7 @@ __global__ void __launch_bounds__(256, kFilterCtas) af_filter_kernel(AfParams p)
             }
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {
-                const int a = (w0 + u) / rounds, i = g0 + (w0 + u - a * rounds) * 256 + (int)threadIdx.x;
+                const int a = (w0 + u) / rounds, round = w0 + u - a * rounds, i = g0 + round * 256 + (int)threadIdx.x;
                 if (a >= n) break;
                 const float T = active_thr[a];
                 int last = 0;
@@ -486,17 +588,27 @@ __global__ void __launch_bounds__(256, kFilterCtas) af_filter_kernel(AfParams p)
                 }
                 // a slot of the list's second half was taken: the next round may not fit
                 if (__syncthreads_or(last >= kListRoom)) {
-                    smooth_listed();
+                    // this part's samples are the list's last
+                    const int listed = n_list;
+                    for (int j = threadIdx.x; j < listed; j += 256)
+                        if (list[j].x == active[a] && (j == 0 || list[j - 1].x != active[a])) part_at = j;
+                    __syncthreads();
+                    dense = 4 * (listed - part_at) >= min(g0 + (round + 1) * 256, g1) - g0;
+                    smooth_listed(dense ? part_at : listed);
                     __syncthreads();
                     if (threadIdx.x == 0) n_list = 0;
                     __syncthreads();
+                    if (dense) {
+                        w1 = a * rounds;
+                        break;
+                    }
                 }
             }
         }
         __syncthreads();  // `active` and its count are read before they are written again
     }
     __syncthreads();
-    smooth_listed();
+    smooth_listed(n_list);
 }
 
 // One thread per frame of the window: can this window's filtered frame
@@ -554,6 +666,7 @@ int af_params(const struct recon_metadata &mr, const float *d_in, float *d_out, 
     p.sup_out = nullptr;
     p.f0 = 0;
     p.f1 = p.P;
+    p.parts = 1;
     if (p.P <= 0 || p.R <= 0 || p.N <= 0) {
         set_error("adaptive filter: empty pull window");
         return CTBB_ERR_ARGUMENT;
@@ -617,7 +730,9 @@ int af_launch(AfParams p, int sup0, int sup1, int smooth0, int smooth1, int thr0
             else af_copy_kernel<false><<<n, 256, 0, stream>>>(p);
             ++launches;
         }
-        const int grid = kParts * std::min(n, num_sms() * kFilterCtas / kParts);
+        p.parts = (int)std::min<size_t>(std::min(kParts, (p.R + 3) / 4),
+                                        std::max<size_t>(1, (size_t)p.R * p.N / kListRoom));
+        const int grid = p.parts * std::min(n, std::max(1, num_sms() * kFilterCtas / p.parts));
         if (vec) af_filter_kernel<true><<<grid, 256, 0, stream>>>(p);
         else af_filter_kernel<false><<<grid, 256, 0, stream>>>(p);
         launches += 1;
