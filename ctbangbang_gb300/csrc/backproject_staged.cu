@@ -555,6 +555,20 @@ bool staged_shape(const BpParams &p, StagedShape *out)
     const float rx = std::fabs(p.x0) + 0.5f * std::fabs(p.pix_x) * (float)p.nx;
     const float ry = std::fabs(p.y0) + 0.5f * std::fabs(p.pix_y) * (float)p.ny;
     if (!(std::sqrt(rx * rx + ry * ry) < 0.9f * p.rf)) return false;
+    // Beyond the column form's windows the alternative is the slice-chunk form.
+    // A visit is staged for whole groups of 8 slices; where the detector spans
+    // fewer, most of that is idle, which small images repay (the slice-chunk
+    // form has too few CTAs for them) and large ones do not.  ms against the
+    // slice-chunk form, by the slices between the detector's edges at the
+    // isocentre and tiles of 16 x 8: 1 slice, 50 tiles 0.55 / 0.89, 120 1.11 /
+    // 1.00, 512 4.26 / 2.68; 3 slices, 50 0.40 / 0.81, 120 0.81 / 0.90, 190
+    // 1.21 / 1.03, 512 3.09 / 2.48; 7 slices, 325 2.08 / 2.29, 512 3.11 / 3.10,
+    // 1152 6.81 / 6.23; 15 slices, 1152 5.24 / 6.05.
+    if (p.nht > kColumnMaxHalfTurns) {
+        const float seen = 2.0f * p.rf * p.tan_cone / p.coll;
+        const long long tiles = (long long)((p.nx + 15) / 16) * ((p.ny + kTileY - 1) / kTileY);
+        if (!(seen >= 12.0f) && tiles > (seen >= 6.0f ? 448 : 96)) return false;
+    }
     struct Candidate {
         int cw, pitch;
     };

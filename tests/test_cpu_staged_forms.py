@@ -114,3 +114,24 @@ def test_tiles_of_tens_of_centimetres(box_check, tmp_path, channels, nx, ny, fov
     spec.recon_fov, spec.x_origin = fov, x0
     visits, outside, misread = _boxes(box_check, spec, tmp_path)
     assert outside == 0 and misread == 0, (visits, outside, misread)
+
+
+def _shape(check, spec, tmp_path):
+    mr = scans.plan_spec(spec, str(tmp_path))
+    L.call("ctbb_update_block_info", C.byref(mr))
+    cw, pitch = C.c_int(-1), C.c_int(-1)
+    assert check.check_staged_shape(C.byref(mr), C.byref(cw), C.byref(pitch)) == 0
+    scans.free_plan(mr)
+    return cw.value, pitch.value
+
+
+# z, raw rows, pitch, pixels, staged; all windows of more than 8 half turns
+WINDOWS = [(0, 2, 1.0, 80, True), (0, 2, 1.0, 120, False), (0, 4, 0.8, 80, True), (0, 4, 0.8, 150, False),
+           (1, 4, 1.0, 256, False), (0, 8, 0.5, 200, True), (0, 8, 0.3, 384, False), (0, 16, 0.25, 384, True)]
+
+
+@pytest.mark.parametrize("z,rows,pitch,pixels,staged", WINDOWS)
+def test_windows_of_many_half_turns(box_check, tmp_path, z, rows, pitch, pixels, staged):
+    """A detector of few slices' height takes the staged form for small images only."""
+    spec = scans.tiny(z, 0, n_rows_raw=rows, n_proj_turn=96, n_channels=128, nx=pixels, ny=pixels, n_slices=4, pitch=pitch)
+    assert (_shape(box_check, spec, tmp_path)[0] > 0) == staged
