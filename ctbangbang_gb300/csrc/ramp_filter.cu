@@ -601,31 +601,34 @@ __global__ void __launch_bounds__(kFftThreads, 4)
     }
 }
 
-// Threads that work on one row pair: one per radix-16 butterfly, at most the
-// CTA.  The CTA's remaining threads take further pairs, each with buffers of
-// its own: a 256-point transform has 16 butterflies to a pass, which left 240
-// of 256 threads idle.  Measured against one pair to a CTA: 9 921 rows of 128
-// samples 56 -> 23 us a call, 20 001 rows of 300 144 -> 90, of 600 212 -> 180,
-// of 960 264 -> 215.
+// Threads that work on one row pair where CTAs are shared: one per
+// radix-16 butterfly, at most the CTA; the CTA's remaining threads take further
+// pairs, each with buffers of its own: a 256-point transform has 16 butterflies
+// to a pass, which left 240 of 256 threads idle.  Measured against one pair to a
+// CTA: 9 921 rows of 128 samples 56 -> 23 us a call, 20 001 rows of 300 144 ->
+// 90, of 600 212 -> 180, of 960 264 -> 215.  Fewer pairs than that get a CTA each,
+// whose threads beyond the butterflies share the loads and stores (SHARED =
+// false; the line is drawn in launch_ramp_filter).
 __host__ __device__ constexpr int pair_threads(int m)
 {
     return m / 16 < 1 ? 1 : (m / 16 < kFftThreads ? m / 16 : kFftThreads);
 }
 
+template <bool SHARED>
 __global__ void __launch_bounds__(kFftThreads, 3) ramp_fft_kernel(FftParams p, const float2 *__restrict__ tw)
 {
     // twiddles come from the read-only cache (one table for every CTA), which
     // leaves shared memory to the transform buffers
     extern __shared__ float2 smem[];
     const int padded = pad(p.m - 1) + 1;
-    const int threads = pair_threads(p.m), groups = kFftThreads / threads;
+    const int threads = SHARED ? pair_threads(p.m) : kFftThreads, groups = SHARED ? kFftThreads / threads : 1;
     const int g = threadIdx.x / threads, t = threadIdx.x - g * threads;
     float2 *buf_a = smem + (size_t)g * 2 * padded;
     float2 *buf_b = buf_a + padded;
     const size_t n_pairs = (p.n_lines + 1) / 2;
     for (size_t pair0 = (size_t)blockIdx.x * groups; pair0 < n_pairs; pair0 += (size_t)gridDim.x * groups) {
         const size_t la = 2 * (pair0 + g), lb = la + 1;
-        const bool has_a = la < p.n_lines, has_b = lb < p.n_lines;
+        const bool has_a = !SHARED || la < p.n_lines, has_b = lb < p.n_lines;
         const float *ra = p.lines + la * (size_t)p.n;
         const float *rb = p.lines + lb * (size_t)p.n;
         __syncthreads();  // previous pairs' stores done before buf_a is rewritten
@@ -809,7 +812,9 @@ int launch_ramp_filter(const RampFilterPlan &plan, float *d_lines, size_t n_line
     const uint64_t bit = dev < 64 ? (uint64_t)1 << dev : 0;
     if (!bit || !(attr_devices.load() & bit)) {
         size_t max_smem = sizeof(float2) * 2 * padded(kMaxRampTransform);
-        CTBB_CUDA_TRY(cudaFuncSetAttribute(ramp_fft_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CTBB_CUDA_TRY(cudaFuncSetAttribute(ramp_fft_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)max_smem));
+        CTBB_CUDA_TRY(cudaFuncSetAttribute(ramp_fft_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)max_smem));
         CTBB_CUDA_TRY(cudaFuncSetAttribute(ramp_fft4096_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)(sizeof(float2) * 2 * padded(kM4096))));
@@ -833,11 +838,18 @@ int launch_ramp_filter(const RampFilterPlan &plan, float *d_lines, size_t n_line
         grid = (int)std::min<size_t>(n_pairs, (size_t)num_sms() * std::min(per_sm, 2));
         ramp_fft4096_kernel<2><<<grid, kFftThreads, smem, stream>>>(p, plan.d_tw16, plan.d_tw16 + 15 * 16);
     } else {
+        // a CTA to a pair while the GPU holds them all at once (three to an
+        // SM): 300 rows of 32 samples take 6 us so and 10 sharing CTAs, of 512
+        // 7 and 12; 1216 rows of 512 14 and 12
         const int groups = kFftThreads / pair_threads(p.m);
-        smem *= groups;
-        per_sm = (int)std::min<size_t>(4, std::max<size_t>(1, (size_t)(220 * 1024) / smem));
-        grid = (int)std::min<size_t>((n_pairs + groups - 1) / groups, (size_t)num_sms() * per_sm);
-        ramp_fft_kernel<<<grid, kFftThreads, smem, stream>>>(p, plan.d_twiddle);
+        const bool shared = groups > 1 && n_pairs > (size_t)num_sms() * 3;
+        if (shared) {
+            smem *= groups;
+            per_sm = (int)std::min<size_t>(4, std::max<size_t>(1, (size_t)(220 * 1024) / smem));
+            grid = (int)std::min<size_t>((n_pairs + groups - 1) / groups, (size_t)num_sms() * per_sm);
+        }
+        auto *kernel = shared ? ramp_fft_kernel<true> : ramp_fft_kernel<false>;
+        kernel<<<grid, kFftThreads, smem, stream>>>(p, plan.d_twiddle);
     }
     count_launch();
     CTBB_CUDA_TRY(cudaGetLastError());
