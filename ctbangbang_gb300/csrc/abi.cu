@@ -82,6 +82,7 @@ struct Context {
     // and per frame of each block window whether that can differ from the union
     DeviceBuffer edge_raw, dirty;
     DeviceRebinTables rebin_tables;
+    CopyError copy_error;  // set by a kernel of this context whose copies did not arrive
     RampFilterPlan ramp;
     RampTcPlan ramp_tc;
     DeviceBuffer tc_work;
@@ -267,12 +268,34 @@ int require_device()
     return CTBB_OK;
 }
 
+// Fails once if a kernel of c found its copies missing (CopyError), in this
+// call or one before it: after the streams that may still set the word have
+// finished, so that it stays clear.
+static int copy_error_check(Context &c)
+{
+    if (!c.copy_error.set()) return CTBB_OK;
+    if (c.prep_stream) CTBB_CUDA_TRY(cudaStreamSynchronize(c.prep_stream));
+    CTBB_CUDA_TRY(cudaStreamSynchronize(c.stream));
+    c.copy_error.clear();
+    set_error("a kernel's wait on a copy into shared memory ran out, in this call or one before it: the result is not "
+              "valid (NaN in its place)");
+    return CTBB_ERR_CUDA;
+}
+
+int *copy_error_word()
+{
+    Context &c = ctx();
+    std::lock_guard<std::mutex> lk(c.mu);
+    return c.copy_error.ensure() == CTBB_OK ? c.copy_error.word : nullptr;
+}
+
 // The adaptive filter on the library-wide stream with the caller's scratch,
 // serialised with the other entry points and counted by the stage profile.
 int run_adaptive_filter_with(const struct recon_metadata &mr, const float *d_in, float *d_out, float *d_scratch)
 {
     Context &c = ctx();
     std::lock_guard<std::mutex> lk(c.mu);
+    CTBB_TRY(copy_error_check(c));
     StageScope scope(c, 0);
     return launch_adaptive_filter(mr, d_in, d_out, d_scratch, c.stream);
 }
@@ -293,7 +316,7 @@ static int do_rebin(Context &c, const struct recon_metadata &mr, const float *d_
     CTBB_TRY(build_rebin_tables(mr, &t));
     CTBB_TRY(upload_rebin_tables(t, &c.rebin_tables, c.stream));
     StageScope scope(c, 1);
-    return launch_rebin(t, c.rebin_tables, d_raw, d_rebin, c.stream);
+    return launch_rebin(t, c.rebin_tables, d_raw, d_rebin, c.copy_error, c.stream);
 }
 
 static int do_filter(Context &c, const struct recon_metadata &mr, float *d_rebin)
@@ -349,7 +372,7 @@ static int do_backproject(Context &c, const struct recon_metadata &mr, const flo
     CTBB_TRY(partial_scratch(c, mr, &part, &part_bytes));
     StageScope scope(c, 3);
     return launch_backproject(mr, t, c.bp_views.as<float4>(), c.bp_theta.as<float>(), c.bp_zpos.as<float>(),
-                              d_rebin, d_block, bp_zpt(), c.stream, nullptr, nullptr, part, part_bytes);
+                              d_rebin, d_block, bp_zpt(), c.copy_error, c.stream, nullptr, nullptr, part, part_bytes);
 }
 
 // The whole-scan paths' backprojection of one block from the context's rows:
@@ -369,7 +392,7 @@ static int backproject_scan_rows(Context &c, const struct recon_metadata &mr, fl
     CTBB_TRY(partial_scratch(c, mr, &part, &part_bytes));
     StageScope scope(c, 3);
     return launch_backproject(mr, t, c.bp_views.as<float4>(), c.bp_theta.as<float>(), c.bp_zpos.as<float>(),
-                              reinterpret_cast<const float *>(c.quads.ptr), d_block, 8, c.stream,
+                              reinterpret_cast<const float *>(c.quads.ptr), d_block, 8, c.copy_error, c.stream,
                               c.qscale.as<float>(), nullptr, part, part_bytes);
 }
 
@@ -478,6 +501,7 @@ static void release_context(Context &c, bool device_sync, bool unbind)
         b->release();
     if (c.rebin_tables.base) cudaFree(c.rebin_tables.base);
     c.rebin_tables = DeviceRebinTables{};
+    c.copy_error.release();
     if (c.ramp.d_spectrum) cudaFree(c.ramp.d_spectrum);
     c.ramp = RampFilterPlan{};
     release_ramp_tc(&c.ramp_tc);
@@ -560,6 +584,7 @@ extern "C" int ctbb_adaptive_filter_device(const struct recon_metadata *mr, cons
     Context &c = ctx();
     CTBB_TRY(require_device(c));
     std::lock_guard<std::mutex> lk(c.mu);
+    CTBB_TRY(copy_error_check(c));
     return do_adaptive(c, *mr, d_in, d_out);
 }
 
@@ -570,7 +595,7 @@ extern "C" int ctbb_rebin_device(const struct recon_metadata *mr, const float *d
     Context &c = ctx();
     CTBB_TRY(require_device(c));
     std::lock_guard<std::mutex> lk(c.mu);
-    CTBB_TRY(copy_error_check());  // of a launch before
+    CTBB_TRY(copy_error_check(c));
     return do_rebin(c, *mr, d_raw, d_rebin);
 }
 
@@ -584,6 +609,7 @@ extern "C" int ctbb_ramp_filter_device(float *d_lines, size_t n_lines, int n_os,
     CTBB_TRY(require_device(ctx()));
     Context &c = ctx();
     std::lock_guard<std::mutex> lk(c.mu);
+    CTBB_TRY(copy_error_check(c));
     CTBB_TRY(prepare_ramp_filter(h_taps, n_os, &c.ramp, c.stream));
     return launch_ramp_filter(c.ramp, d_lines, n_lines, c.stream);
 }
@@ -607,6 +633,7 @@ extern "C" int ctbb_ramp_filter_fp16_device(const float *d_lines, size_t n_lines
     Context &c = ctx();
     CTBB_TRY(require_device(c));
     std::lock_guard<std::mutex> lk(c.mu);
+    CTBB_TRY(copy_error_check(c));
     CTBB_TRY(prepare_ramp_tc(h_taps, n_os, &c.ramp_tc, c.stream));
     CTBB_TRY(c.tc_work.ensure(ramp_tc_work_bytes(n_lines, n_os)));
     StageScope scope(c, 2);
@@ -627,6 +654,7 @@ extern "C" int ctbb_backproject_fp16_device(const struct recon_metadata *mr, con
     Context &c = ctx();
     CTBB_TRY(require_device(c));
     std::lock_guard<std::mutex> lk(c.mu);
+    CTBB_TRY(copy_error_check(c));
     BackprojectTables t;
     CTBB_TRY(build_backproject_tables(*mr, &t));
     CTBB_TRY(upload(c.bp_views, t.views, c.stream));
@@ -637,8 +665,8 @@ extern "C" int ctbb_backproject_fp16_device(const struct recon_metadata *mr, con
     CTBB_TRY(partial_scratch(c, *mr, &part, &part_bytes));
     StageScope scope(c, 3);
     return launch_backproject(*mr, t, c.bp_views.as<float4>(), c.bp_theta.as<float>(), c.bp_zpos.as<float>(),
-                              static_cast<const float *>(d_quads), d_block, 8, c.stream, d_scale, nullptr, part,
-                              part_bytes);
+                              static_cast<const float *>(d_quads), d_block, 8, c.copy_error, c.stream, d_scale,
+                              nullptr, part, part_bytes);
 }
 
 extern "C" int ctbb_backproject_device(const struct recon_metadata *mr, const float *d_rebin, float *d_block)
@@ -648,7 +676,7 @@ extern "C" int ctbb_backproject_device(const struct recon_metadata *mr, const fl
     Context &c = ctx();
     CTBB_TRY(require_device(c));
     std::lock_guard<std::mutex> lk(c.mu);
-    CTBB_TRY(copy_error_check());  // of a launch before
+    CTBB_TRY(copy_error_check(c));
     return do_backproject(c, *mr, d_rebin, d_block);
 }
 
@@ -660,6 +688,7 @@ extern "C" int ctbb_finalize_device(const struct recon_metadata *mr, const float
     Context &c = ctx();
     CTBB_TRY(require_device(c));
     std::lock_guard<std::mutex> lk(c.mu);
+    CTBB_TRY(copy_error_check(c));
     return do_finalize(c, *mr, d_image, d_final, mu_water);
 }
 
@@ -698,7 +727,9 @@ static int drained(Context &c, Body &&body)
                   cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
         return CTBB_ERR_CUDA;
     }
-    return st == CTBB_OK ? copy_error_check() : st;
+    if (st == CTBB_OK) return copy_error_check(c);
+    c.copy_error.clear();  // this call fails already
+    return st;
 }
 
 static int reconstruct_device_in(Context &c, struct recon_metadata *mr, const float *d_scan, float *d_final,
@@ -957,7 +988,8 @@ static int run_edge_patch(Context &c, const struct recon_metadata &mb, const Reb
         float *d_out = c.rebin.as<float>() + (patch_view + slot) * view_elems - (size_t)r.first * view_elems;
         {
             StageScope scope(c, 1);
-            CTBB_TRY(launch_rebin(tb, c.rebin_tables, c.edge_raw.as<float>(), d_out, c.stream, r.first, r.second));
+            CTBB_TRY(launch_rebin(tb, c.rebin_tables, c.edge_raw.as<float>(), d_out, c.copy_error, c.stream,
+                                  r.first, r.second));
         }
         const size_t n = (size_t)(r.second - r.first);
         CTBB_TRY(filter_scan_rows(c, (patch_view + slot) * d.n_rows, n * d.n_rows, (int)d.n_rows, (int)d.n_os));
@@ -1075,7 +1107,7 @@ static int prepare_scan_device(Context &c, struct recon_metadata *mr, const floa
     CTBB_TRY(upload_rebin_tables(rt, &c.rebin_tables, c.stream));
     {
         StageScope scope(c, 1);
-        CTBB_TRY(launch_rebin(rt, c.rebin_tables, c.raw_filt.as<float>(), c.rebin.as<float>(), c.stream));
+        CTBB_TRY(launch_rebin(rt, c.rebin_tables, c.raw_filt.as<float>(), c.rebin.as<float>(), c.copy_error, c.stream));
     }
     // each block's edge frames that can filter differently from the union
     for (size_t b = 0; b < blocks.size(); ++b) {
@@ -1211,7 +1243,7 @@ static int tuned_shape(Context &c, const BpParams &p_any, const BpShape &fallbac
         const size_t part = backproject_partial_bytes(p, cand[k]);
         if (part) CTBB_TRY(c.bp_partial.ensure(part));
         auto launch = [&]() {
-            return launch_backproject_params(p, cand[k], c.stream, c.bp_partial.ptr, c.bp_partial.bytes);
+            return launch_backproject_params(p, cand[k], c.copy_error, c.stream, c.bp_partial.ptr, c.bp_partial.bytes);
         };
         CTBB_TRY(launch());  // warm-up (module load, caches)
         float ms = 1e30f;
@@ -1269,7 +1301,7 @@ static int reconstruct_scan_device_in(Context &c, struct recon_metadata *mr, con
             const size_t part = backproject_partial_bytes(p, shape);
             if (part) CTBB_TRY(c.bp_partial.ensure(part));
             StageScope scope(c, 3);
-            CTBB_TRY(launch_backproject_params(p, shape, c.stream, c.bp_partial.ptr, c.bp_partial.bytes));
+            CTBB_TRY(launch_backproject_params(p, shape, c.copy_error, c.stream, c.bp_partial.ptr, c.bp_partial.bytes));
         }
         CTBB_TRY(do_finalize(c, *mr, c.image.as<float>(), d_final, mu_water));
         CTBB_CUDA_TRY(cudaStreamSynchronize(c.stream));
@@ -1389,7 +1421,8 @@ extern "C" int ctbb_batch_run(void)
                 if (it.first == sh) group.push_back(it.second);
             CTBB_TRY(g_batch_params.ensure(backproject_batch_bytes(group.size())));
             StageScope scope(c, 3);
-            CTBB_TRY(launch_backproject_batch(group, sh, g_batch_params.ptr, g_batch_params.bytes, c.stream));
+            CTBB_TRY(launch_backproject_batch(group, sh, g_batch_params.ptr, g_batch_params.bytes, c.copy_error,
+                                              c.stream));
         }
         for (size_t s = 0; s < g_batch.size(); ++s)
             CTBB_TRY(do_finalize(c, *g_batch[s].mr, g_slots[s].image.as<float>(), g_batch[s].d_final,
@@ -1489,6 +1522,7 @@ extern "C" int ctbb_adaptive_filter_kk(struct recon_metadata *mr)
     CTBB_TRY(require_device(ctx()));
     Context &c = ctx();
     std::lock_guard<std::mutex> lk(c.mu);
+    CTBB_TRY(copy_error_check(c));
     BlockDims d = block_dims(*mr);
     size_t bytes = d.raw_elems() * sizeof(float);
     CTBB_TRY(c.raw_in.ensure(bytes));
@@ -1529,7 +1563,7 @@ extern "C" int ctbb_rebin_filter(struct recon_metadata *mr)
     if (mr->flags.testing && mr->ctd.rebin)
         CTBB_CUDA_TRY(cudaMemcpyAsync(mr->ctd.rebin, d_rebin, rebin_bytes, cudaMemcpyDeviceToHost, c.stream));
     CTBB_CUDA_TRY(cudaStreamSynchronize(c.stream));
-    return copy_error_check();
+    return copy_error_check(c);
 }
 
 extern "C" int ctbb_backproject(struct recon_metadata *mr)
@@ -1558,7 +1592,7 @@ extern "C" int ctbb_backproject(struct recon_metadata *mr)
     CTBB_CUDA_TRY(cudaFree(mr->ctd.d_rebin));
     if (c.our_d_rebin == mr->ctd.d_rebin) c.our_d_rebin = nullptr;
     mr->ctd.d_rebin = nullptr;
-    return copy_error_check();
+    return copy_error_check(c);
 }
 
 static int finalize_common(struct recon_metadata *mr, float mu_water)
@@ -1581,6 +1615,7 @@ static int finalize_common(struct recon_metadata *mr, float mu_water)
     CTBB_TRY(require_device(ctx()));
     Context &c = ctx();
     std::lock_guard<std::mutex> lk(c.mu);
+    CTBB_TRY(copy_error_check(c));
     size_t plane = (size_t)mr->rp.nx * mr->rp.ny;
     size_t n_img = plane * mr->ri.n_slices_recon;
     int n_final = ctbb_n_slices_final(mr);
@@ -1796,8 +1831,8 @@ static int scan_streamed(Context &c, struct recon_metadata *mr, ChunkFeed &feed,
             if (v_ready > v_done) {
                 {
                     StageScope scope(c, 1);
-                    status = launch_rebin(rt, c.rebin_tables, c.raw_filt.as<float>(), c.rebin.as<float>(), c.stream,
-                                          v_done, v_ready);
+                    status = launch_rebin(rt, c.rebin_tables, c.raw_filt.as<float>(), c.rebin.as<float>(), c.copy_error,
+                                          c.stream, v_done, v_ready);
                 }
                 if (status != CTBB_OK) break;
                 status = filter_scan_rows(c, (size_t)v_done * dg.n_rows, (size_t)(v_ready - v_done) * dg.n_rows,

@@ -1173,7 +1173,8 @@ size_t backproject_partial_bytes(const BpParams &p, const BpShape &shape)
     return chunks <= 1 ? 0 : (size_t)chunks * p.n_slices * p.nx * p.ny * sizeof(float);
 }
 
-int launch_backproject_params(const BpParams &p_in, const BpShape &shape, cudaStream_t stream, void *scratch,
+int launch_backproject_params(const BpParams &p_in, const BpShape &shape, CopyError &errors, cudaStream_t stream,
+                              void *scratch,
                               size_t scratch_bytes)
 {
     BpParams p = p_in;
@@ -1187,7 +1188,7 @@ int launch_backproject_params(const BpParams &p_in, const BpShape &shape, cudaSt
     }
     StagedShape st;
     if (shape.staged && staged_shape(p, &st)) {
-        CTBB_TRY(launch_backproject_staged(p, st, stream));
+        CTBB_TRY(launch_backproject_staged(p, st, errors, stream));
         return p.partial ? launch_combine(p, stream) : CTBB_OK;
     }
     const bool quad = p.vscale != nullptr;
@@ -1236,13 +1237,13 @@ int launch_backproject_params(const BpParams &p_in, const BpShape &shape, cudaSt
 
 int launch_backproject(const struct recon_metadata &mr, const BackprojectTables &t,
                        const float4 *d_views, const float *d_theta, const float *d_zpos, const float *d_rebin,
-                       float *d_block, int zpt, cudaStream_t stream, const float *d_vscale, const BpShape *shape,
-                       void *scratch, size_t scratch_bytes)
+                       float *d_block, int zpt, CopyError &errors, cudaStream_t stream, const float *d_vscale,
+                       const BpShape *shape, void *scratch, size_t scratch_bytes)
 {
     const BpShape s = shape ? fit_bp_shape(*shape, t.nht) : window_bp_shape(zpt, d_vscale != nullptr, t.nht);
     BpParams p;
     CTBB_TRY(make_backproject_params(mr, t, d_views, d_theta, d_zpos, d_rebin, d_block, d_vscale, s, &p));
-    return launch_backproject_params(p, s, stream, scratch, scratch_bytes);
+    return launch_backproject_params(p, s, errors, stream, scratch, scratch_bytes);
 }
 
 // the blocks' TMA descriptors first (aligned by the allocation), then their
@@ -1257,7 +1258,7 @@ namespace {
 // The blocks of a batch that take the staged form: those of one staged shape
 // together, one launch per angle chunk.
 int launch_staged_batch(const std::vector<BpParams> &blocks, int chunks, void *d_buf, size_t buf_bytes,
-                        cudaStream_t stream)
+                        CopyError &errors, cudaStream_t stream)
 {
     std::vector<StagedShape> shapes(blocks.size());
     std::vector<StagedShape> kinds;
@@ -1301,7 +1302,7 @@ int launch_staged_batch(const std::vector<BpParams> &blocks, int chunks, void *d
                                       stream));
         for (int ac = 0; ac < n_ac; ++ac)
             CTBB_TRY(launch_backproject_staged_batch(d_params, d_start, d_maps, start.back(), (int)group.size(), ac,
-                                                     n_ac, kind, stream));
+                                                     n_ac, kind, errors, stream));
     }
     return CTBB_OK;
 }
@@ -1309,10 +1310,10 @@ int launch_staged_batch(const std::vector<BpParams> &blocks, int chunks, void *d
 }  // namespace
 
 int launch_backproject_batch(const std::vector<BpParams> &blocks, const BpShape &shape, void *d_buf, size_t buf_bytes,
-                             cudaStream_t stream)
+                             CopyError &errors, cudaStream_t stream)
 {
     if (blocks.empty()) return CTBB_OK;
-    if (shape.staged) return launch_staged_batch(blocks, shape.staged, d_buf, buf_bytes, stream);
+    if (shape.staged) return launch_staged_batch(blocks, shape.staged, d_buf, buf_bytes, errors, stream);
     const bool quad = blocks[0].vscale != nullptr;
     for (const BpParams &p : blocks)
         if ((p.vscale != nullptr) != quad || p.nos != blocks[0].nos) {

@@ -25,6 +25,8 @@ struct BackprojectTables {
     void set_view_row(int i, int k, unsigned row);
 };
 
+struct CopyError;  // tma.cuh: a context's word for copies that did not arrive
+
 // Kernel parameters of one block's backprojection.
 struct BpParams {
     const float *rebin;    // [V][R][Nos] float32, or footprint quads [V][R][Nos][4] FP16
@@ -94,12 +96,12 @@ struct StagedShape {
 // not apply (FP16 footprint words, rows off 16-byte boundaries, pixels whose footprint is too wide,
 // more than 32 slices, voxels near the source's circle).
 bool staged_shape(const BpParams &p, StagedShape *out);
-int launch_backproject_staged(const BpParams &p, const StagedShape &s, cudaStream_t stream);
+int launch_backproject_staged(const BpParams &p, const StagedShape &s, CopyError &errors, cudaStream_t stream);
 // Angle chunk ac of n_ac of n blocks of one staged shape, total CTA tiles.
 // d_maps: the blocks' TMA descriptors (staged_map, staged_map_bytes() each, 64-byte aligned).
 int launch_backproject_staged_batch(const BpParams *d_params, const unsigned *d_start, const void *d_maps,
                                     unsigned total, int n, int ac, int n_ac, const StagedShape &s,
-                                    cudaStream_t stream);
+                                    CopyError &errors, cudaStream_t stream);
 size_t staged_map_bytes();
 int staged_map(const BpParams &p, const StagedShape &s, void *out);
 unsigned staged_tiles(const BpParams &p, const StagedShape &s);
@@ -130,8 +132,8 @@ int make_backproject_params(const struct recon_metadata &mr, const BackprojectTa
                             const float *d_vscale, const BpShape &shape, BpParams *p);
 // scratch: device memory for the partial image sums of shape.achunks > 1
 // (backproject_partial_bytes); with less, the angles run as one chunk.
-int launch_backproject_params(const BpParams &p, const BpShape &shape, cudaStream_t stream, void *scratch = nullptr,
-                              size_t scratch_bytes = 0);
+int launch_backproject_params(const BpParams &p, const BpShape &shape, CopyError &errors, cudaStream_t stream,
+                              void *scratch = nullptr, size_t scratch_bytes = 0);
 // Bytes of partial image sums a launch of this shape needs (0: none).
 size_t backproject_partial_bytes(const BpParams &p, const BpShape &shape);
 // Device bytes launch_backproject_batch needs for n blocks' parameters.
@@ -141,11 +143,11 @@ size_t backproject_batch_bytes(size_t n_blocks);
 // to the blocks' images in chunk order; d_buf holds
 // backproject_batch_bytes(blocks.size()).
 int launch_backproject_batch(const std::vector<BpParams> &blocks, const BpShape &shape, void *d_buf,
-                             size_t buf_bytes, cudaStream_t stream);
+                             size_t buf_bytes, CopyError &errors, cudaStream_t stream);
 int launch_backproject(const struct recon_metadata &mr, const BackprojectTables &t,
                        const float4 *d_views, const float *d_theta, const float *d_zpos, const float *d_rebin,
-                       float *d_block, int zpt, cudaStream_t stream, const float *d_vscale = nullptr,
-                       const BpShape *shape = nullptr, void *scratch = nullptr, size_t scratch_bytes = 0);
+                       float *d_block, int zpt, CopyError &errors, cudaStream_t stream,
+                       const float *d_vscale = nullptr, const BpShape *shape = nullptr, void *scratch = nullptr, size_t scratch_bytes = 0);
 // d_vscale non-null: d_rebin holds footprint quads [V][R][Nos][4] FP16 (the
 // reduced-storage rows, see ramp_tc.h) with view v's scale at d_vscale[v R].
 

@@ -444,10 +444,12 @@ __device__ __forceinline__ void backproject_staged_tile(const Params &p, int bx,
         if (!alive) break;
     }
     if (!alive) {
-        // a wait ran out: report it and leave
+        // a wait ran out: report it, and no image in place of a part of one
         *reinterpret_cast<volatile int *>(error) = 1;
         wait_for_stray_copies();
-        return;
+#pragma unroll
+        for (int m = 0; m < kSub / 2; ++m)
+            img[m] = make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
     }
     if (!inside) return;
     const size_t plane = (size_t)p.nx * p.ny;
@@ -614,10 +616,10 @@ bool staged_shape(const BpParams &p, StagedShape *out)
     return false;
 }
 
-int launch_backproject_staged(const BpParams &p, const StagedShape &s, cudaStream_t stream)
+int launch_backproject_staged(const BpParams &p, const StagedShape &s, CopyError &errors, cudaStream_t stream)
 {
-    int *err = copy_error_word();
-    if (!err) return CTBB_ERR_ALLOC;
+    CTBB_TRY(errors.ensure());
+    int *err = errors.word;
     const dim3 grid((p.nx + tile_x(s.cw) - 1) / tile_x(s.cw), (p.ny + kTileY - 1) / kTileY, std::max(p.n_achunks, 1));
     return with_staged(s, [&](auto cw, auto pitch) -> int {
         constexpr int CW = decltype(cw)::value, PITCH = decltype(pitch)::value;
@@ -651,10 +653,10 @@ int staged_map(const BpParams &p, const StagedShape &s, void *out)
 
 int launch_backproject_staged_batch(const BpParams *d_params, const unsigned *d_start, const void *d_maps,
                                     unsigned total, int n, int ac, int n_ac, const StagedShape &s,
-                                    cudaStream_t stream)
+                                    CopyError &errors, cudaStream_t stream)
 {
-    int *err = copy_error_word();
-    if (!err) return CTBB_ERR_ALLOC;
+    CTBB_TRY(errors.ensure());
+    int *err = errors.word;
     return with_staged(s, [&](auto cw, auto pitch) -> int {
         constexpr int CW = decltype(cw)::value, PITCH = decltype(pitch)::value;
         const StagedLayout lay = staged_layout(CW, s.half_bytes);

@@ -558,16 +558,21 @@ __global__ void __launch_bounds__(128) rebin_staged_kernel(RebinParams p, Staged
             b1 = box - f0[0] * kFrame + tap.i1 - tile.ch0;
         }
     }
-    if (!barrier_wait(bar, 0)) {
-        *reinterpret_cast<volatile int *>(error) = 1;
-        wait_for_stray_copies();
-        return;
-    }
-    if (!in) return;
+    const bool copied = barrier_wait(bar, 0);
     const bool z_ffs = TWO ? p.n_ffs == 4 : p.n_ffs == 2;
     const size_t nos = (size_t)p.Nos;
     const int out_first = z_ffs ? 2 * r0 + (p.reverse_rows ? 1 - side : side) : r0;
     const size_t out_step = (z_ffs ? 2 : 1) * nos;
+    if (!copied) {
+        *reinterpret_cast<volatile int *>(error) = 1;
+        wait_for_stray_copies();
+        if (in)
+            for (int v = w0; v < w1; ++v)
+                for (int r = 0; r < n_rows; ++r)
+                    p.out[((size_t)v * p.R + out_first) * nos + c + r * out_step] = __int_as_float(0x7fffffff);
+        return;
+    }
+    if (!in) return;
     for (int v = w0; v < w1; ++v) {
         const int proj = v + p.add;
         int i0, i1, j0 = 0, j1 = 0;
@@ -622,7 +627,7 @@ int staged_frames(const RebinTables &t, const float *d_raw, int spots, int *chan
 }
 
 int launch_rebin_staged(const RebinTables &t, const DeviceRebinTables &dt, const RebinParams &p, bool two, int frames,
-                        int channels, cudaStream_t stream)
+                        int channels, CopyError &errors, cudaStream_t stream)
 {
     const cuuint64_t row = (cuuint64_t)t.n_channels * 4, frame = row * t.n_rows_raw;
     const cuuint64_t dims[4] = {(cuuint64_t)t.n_channels, (cuuint64_t)t.n_rows_raw, (cuuint64_t)t.n_ffs,
@@ -631,8 +636,8 @@ int launch_rebin_staged(const RebinTables &t, const DeviceRebinTables &dt, const
     const cuuint32_t box[4] = {(cuuint32_t)channels, kRowsPerThread, 1, (cuuint32_t)frames};
     CUtensorMap map;
     CTBB_TRY(tensor_map_f32(&map, p.raw, 4, dims, strides, box));
-    int *err = copy_error_word();
-    if (!err) return CTBB_ERR_ALLOC;
+    CTBB_TRY(errors.ensure());
+    int *err = errors.word;
     StagedRebin g;
     g.tiles = dt.tiles;
     g.n_tiles = (t.n_os + kRebinTile - 1) / kRebinTile;
@@ -664,7 +669,7 @@ int rebin_frames_needed(const RebinTables &t, int v)
 }
 
 int launch_rebin(const RebinTables &t, const DeviceRebinTables &dt, const float *d_raw,
-                 float *d_out, cudaStream_t stream, int v_begin, int v_end)
+                 float *d_out, CopyError &errors, cudaStream_t stream, int v_begin, int v_end)
 {
     if (v_end < 0 || v_end > t.n_views) v_end = t.n_views;
     if (v_begin < 0) v_begin = 0;
@@ -696,7 +701,7 @@ int launch_rebin(const RebinTables &t, const DeviceRebinTables &dt, const float 
     const bool bilinear = t.mode == RebinMode::kNoFfs || t.mode == RebinMode::kZFfs;
     int channels = 0;
     if (const int frames = staged_frames(t, d_raw, bilinear ? 1 : 2, &channels))
-        return launch_rebin_staged(t, dt, p, !bilinear, frames, channels, stream);
+        return launch_rebin_staged(t, dt, p, !bilinear, frames, channels, errors, stream);
     size_t n_raw = (size_t)t.n_ffs * t.n_proj * t.n_rows_raw * t.n_channels;
     size_t n_out = (size_t)t.n_views * t.n_rows * t.n_os;
     bool narrow = n_raw < ((size_t)1 << 31) && n_out < ((size_t)1 << 31);

@@ -46,6 +46,8 @@ struct RebinTables {
     std::vector<float> focal_offset; // d_alpha_r * n_proj_ffs / (2 pi) per focal spot
 };
 
+struct CopyError;  // tma.cuh: a context's word for copies that did not arrive
+
 struct DeviceRebinTables {
     void *base = nullptr;
     size_t capacity = 0;
@@ -77,7 +79,7 @@ int staged_frames(const RebinTables &t, const float *d_raw, int spots, int *chan
 int upload_rebin_tables(const RebinTables &t, DeviceRebinTables *dt, cudaStream_t stream);
 // Views [v_begin, v_end) of the output (v_end < 0: all views).
 int launch_rebin(const RebinTables &t, const DeviceRebinTables &dt, const float *d_raw,
-                 float *d_out, cudaStream_t stream, int v_begin = 0, int v_end = -1);
+                 float *d_out, CopyError &errors, cudaStream_t stream, int v_begin = 0, int v_end = -1);
 // Frames of the pull window view v reads (focal-spot frames of the view-axis
 // taps of every channel): all lie below rebin_frames_needed(t, v).
 int rebin_frames_needed(const RebinTables &t, int v);

@@ -1,6 +1,4 @@
 // tma.cu -- host side of tma.cuh.
-#include <mutex>
-
 #include "tma.cuh"
 
 namespace ctbb {
@@ -32,31 +30,25 @@ int tensor_map_f32(CUtensorMap *map, const float *base, int rank, const cuuint64
     return CTBB_OK;
 }
 
-int *copy_error_word()
+int CopyError::ensure()
 {
-    static std::once_flag once;
-    static int *word = nullptr;
-    std::call_once(once, [] {
-        void *v = nullptr;
-        if (cudaHostAlloc(&v, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
-            word = static_cast<int *>(v);
-            *word = 0;
-        } else {
-            cudaGetLastError();
-            set_error("no pinned memory for the kernels' error word");
-        }
-    });
-    return word;
+    if (word) return CTBB_OK;
+    void *v = nullptr;
+    const cudaError_t e = cudaHostAlloc(&v, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        set_error("no pinned memory for the kernels' error word: %s", cudaGetErrorString(e));
+        return CTBB_ERR_ALLOC;
+    }
+    word = static_cast<int *>(v);
+    *word = 0;
+    return CTBB_OK;
 }
 
-int copy_error_check()
+void CopyError::release()
 {
-    int *w = copy_error_word();
-    if (w && *reinterpret_cast<volatile int *>(w)) {
-        set_error("a kernel's wait on a copy into shared memory ran out; the result is not valid");
-        return CTBB_ERR_CUDA;
-    }
-    return CTBB_OK;
+    if (word) cudaFreeHost(word);
+    word = nullptr;
 }
 
 }  // namespace ctbb

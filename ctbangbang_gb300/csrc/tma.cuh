@@ -1,6 +1,6 @@
 // tma.cuh -- bulk tensor copies into shared memory: the mbarrier helpers, the
-// descriptor of a float32 tensor, and the word a kernel sets when one of its
-// bounded waits runs out.
+// descriptor of a float32 tensor, and the word a context's kernels set when one
+// of their bounded waits runs out.
 #pragma once
 
 #include <cuda.h>
@@ -16,12 +16,21 @@ namespace ctbb {
 // dims 1 .. rank - 1 in bytes); samples outside it read as zeros.
 int tensor_map_f32(CUtensorMap *map, const float *base, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
                    const cuuint32_t *box);
-// The word kernels set when a bounded wait runs out, in pinned host memory so
-// that it is read without a copy; null if it could not be allocated.
+// The word that the kernels of one context set when a bounded wait on a copy
+// runs out, in pinned host memory so that it is read without a copy.  Such a
+// kernel also writes NaN in place of the results it could not form.  Every
+// stage call of the context looks at the word before its own launches, every
+// synchronising call after its last; the first to find it set clears it and
+// fails.
+struct CopyError {
+    int *word = nullptr;
+    int ensure();  // CTBB_ERR_ALLOC if there is no pinned memory
+    bool set() const { return word && *const_cast<volatile int *>(word); }
+    void clear() { if (word) *const_cast<volatile int *>(word) = 0; }
+    void release();
+};
+// The library-wide context's word (allocated if need be).
 int *copy_error_word();
-// CTBB_ERR_CUDA once a kernel's bounded wait has run out (read after a stream
-// synchronisation, or at the next call).
-int copy_error_check();
 
 namespace {
 

@@ -306,6 +306,13 @@ int ctbb_finalize_image_stack_hu(struct recon_metadata *mr, float mu_water);
 /* library stream).  These are what the drop-in functions call.              */
 /* ------------------------------------------------------------------------- */
 
+/* The rebin and backprojection kernels copy detector samples to shared memory
+   with a bounded wait.  Should one run out (two seconds; it takes a faulty
+   device), the kernel writes NaN where its results belong, and one call of
+   that context fails with CTBB_ERR_CUDA: the synchronising call that launched
+   it, or for the asynchronous stages the next call after it.  A program whose
+   last call is a stage finds the NaN in its output. */
+
 /* Adaptive filter of one pull window: d_raw_in -> d_raw_out (distinct buffers,
    [n_proj_pull][n_rows_raw][n_channels]).  Uses mr->cg, mr->ri, mr->rp. */
 int ctbb_adaptive_filter_device(const struct recon_metadata *mr,
