@@ -68,7 +68,7 @@ constexpr int kTileB = BN * BK * 2;  // bytes of one B tile (32 KiB)
 constexpr int kStageBytes = 2 * kTileA + 2 * kTileB;
 constexpr int kSmemBytes = kStages * kStageBytes + 1024 /* alignment */ + 256 /* barriers */;
 constexpr int kNPad = 1536;          // T padded to a whole number of 256-sample tiles
-constexpr int kMaxTiles = kNPad / (BN - 1);  // output tiles of a row
+constexpr int kMaxTiles = (kNPad + BN - 2) / (BN - 1);  // output tiles of a row (footprint words: 255 columns each)
 constexpr uint32_t kWaitLimit = 1u << 30;
 constexpr uint64_t kWaitNs = 2000000000ull;  // 2 s
 
@@ -750,10 +750,9 @@ int launch_ramp_tc(const RampTcPlan &plan, const float *d_rows, size_t n_lines, 
     p.rows_per_view = rows_per_view > 0 ? rows_per_view : BM;
     const int step = quad ? tile_step<true>() : tile_step<false>();
     dim3 grid((n + step - 1) / step, (unsigned)((n_lines + BM - 1) / BM));
-    if ((grid.x - 1) * step + BN > kNPad) {
-        set_error("ramp filter (tensor cores): row length %d beyond the padded kernel", n);
-        return CTBB_ERR_ARGUMENT;
-    }
+    // a last tile that ends past the padded taps (footprint words of 1536
+    // samples) computes zeros there: the taps' map fills with them
+    static_assert(kMaxTiles * (BN - 1) >= kNPad, "an order for every tile");
     // K order: the slices of the row farthest from the tile's outputs first.
     // Near the diagonal the taps are large (the centre tap and its odd
     // neighbours, which cancel it to a small output); far ones sum to about
