@@ -1255,37 +1255,47 @@ size_t backproject_batch_bytes(size_t n_blocks)
 
 namespace {
 
+// The angle chunks a launch of this block alone splits its angles into, limit
+// at most.
+int staged_block_chunks(const BpParams &p, const StagedShape &s, int limit)
+{
+    const int chunks = staged_chunks(p, s, limit);
+    return chunks <= p.n_half ? chunks : 1;
+}
+
 // The blocks of a batch that take the staged form: those of one staged shape
-// together, one launch per angle chunk.
-int launch_staged_batch(const std::vector<BpParams> &blocks, int chunks, void *d_buf, size_t buf_bytes,
+// and one number of angle chunks together, one launch per chunk.  A block has
+// the chunks it has alone, so that its image is the same sum.
+int launch_staged_batch(const std::vector<BpParams> &blocks, int limit, void *d_buf, size_t buf_bytes,
                         CopyError &errors, cudaStream_t stream)
 {
-    std::vector<StagedShape> shapes(blocks.size());
-    std::vector<StagedShape> kinds;
+    using Kind = std::pair<StagedShape, int>;
+    std::vector<Kind> kind_of(blocks.size()), kinds;
     for (size_t b = 0; b < blocks.size(); ++b) {
-        if (!staged_shape(blocks[b], &shapes[b])) {
+        if (!staged_shape(blocks[b], &kind_of[b].first)) {
             set_error("backproject batch: a block does not fit the staged form");
             return CTBB_ERR_ARGUMENT;
         }
-        if (std::find(kinds.begin(), kinds.end(), shapes[b]) == kinds.end()) kinds.push_back(shapes[b]);
+        kind_of[b].second = staged_block_chunks(blocks[b], kind_of[b].first, limit);
+        if (std::find(kinds.begin(), kinds.end(), kind_of[b]) == kinds.end()) kinds.push_back(kind_of[b]);
     }
     if (backproject_batch_bytes(blocks.size()) > buf_bytes) {
         set_error("backproject batch: parameter buffer too small");
         return CTBB_ERR_ARGUMENT;
     }
-    for (const StagedShape &kind : kinds) {
+    for (const Kind &kind : kinds) {
+        const StagedShape &shape = kind.first;
+        const int n_ac = kind.second;
         std::vector<BpParams> group;
         std::vector<unsigned> start(1, 0);
         std::vector<unsigned char> maps;
-        int n_ac = std::max(1, chunks);
         for (size_t b = 0; b < blocks.size(); ++b) {
-            if (!(shapes[b] == kind)) continue;
+            if (!(kind_of[b] == kind)) continue;
             group.push_back(blocks[b]);
             alignas(64) unsigned char map[256];
-            CTBB_TRY(staged_map(blocks[b], kind, map));
+            CTBB_TRY(staged_map(blocks[b], shape, map));
             maps.insert(maps.end(), map, map + staged_map_bytes());
-            n_ac = std::min(n_ac, blocks[b].n_half);
-            const unsigned long long next = (unsigned long long)start.back() + staged_tiles(blocks[b], kind);
+            const unsigned long long next = (unsigned long long)start.back() + staged_tiles(blocks[b], shape);
             if (next >= (1ull << 31)) {
                 set_error("backproject batch: more than 2^31 CTA tiles");
                 return CTBB_ERR_ARGUMENT;
@@ -1302,7 +1312,7 @@ int launch_staged_batch(const std::vector<BpParams> &blocks, int chunks, void *d
                                       stream));
         for (int ac = 0; ac < n_ac; ++ac)
             CTBB_TRY(launch_backproject_staged_batch(d_params, d_start, d_maps, start.back(), (int)group.size(), ac,
-                                                     n_ac, kind, errors, stream));
+                                                     n_ac, shape, errors, stream));
     }
     return CTBB_OK;
 }
