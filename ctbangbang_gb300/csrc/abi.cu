@@ -1178,17 +1178,20 @@ static int prepared_block_params(Context &c, const struct recon_metadata &mb, co
 // ---- autotuner -------------------------------------------------------------
 // Picks a backprojector launch shape (slices per thread, CTA size, CTAs per
 // SM, CTA width) for each geometry class -- image size, slices per block, row
-// length, detector rows, half turns, row storage -- by timing every candidate
-// once on the first block of that class (CUDA events on the context's
-// stream; the block is recomputed by the chosen shape afterwards), and caches
-// the choice for the process.
+// length, detector rows, half turns, row storage, the staged form's tile -- by
+// timing every candidate once on the first block of that class (CUDA events on
+// the context's stream; the block is recomputed by the chosen shape
+// afterwards), and caches the choice for the process.
 
 struct TuneKey {
-    int nx, ny, n_slices, nos, n_rows, nht, quad, staged;  // staged: the staged form applies
+    int nx, ny, n_slices, nos, n_rows, nht, quad;
+    int staged_cw, staged_pitch;  // the staged form's tile, which the pixel size decides (0: another form)
+    unsigned staged_bytes;
     bool operator<(const TuneKey &o) const
     {
-        return std::tie(nx, ny, n_slices, nos, n_rows, nht, quad, staged) <
-               std::tie(o.nx, o.ny, o.n_slices, o.nos, o.n_rows, o.nht, o.quad, o.staged);
+        return std::tie(nx, ny, n_slices, nos, n_rows, nht, quad, staged_cw, staged_pitch, staged_bytes) <
+               std::tie(o.nx, o.ny, o.n_slices, o.nos, o.n_rows, o.nht, o.quad, o.staged_cw, o.staged_pitch,
+                        o.staged_bytes);
     }
 };
 
@@ -1218,7 +1221,7 @@ static int tuned_shape(Context &c, const BpParams &p_any, const BpShape &fallbac
     StagedShape st;
     const bool staged = staged_shape(p_any, &st);
     const TuneKey key{p_any.nx, p_any.ny, p_any.n_slices, p_any.nos, p_any.n_rows, p_any.nht, quad ? 1 : 0,
-                      staged ? 1 : 0};
+                      staged ? st.cw : 0, staged ? st.pitch : 0, staged ? st.half_bytes : 0u};
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tuned.find(key);

@@ -53,3 +53,23 @@ def test_batch_equals_tuned_scan_alone(lib, tmp_path, kinds):
         L.call("ctbb_set_autotune", 0)
         for s in batch:
             s.close()
+
+
+def test_autotuner_times_each_tile(lib, tmp_path):
+    """Two fields of view of the same counts run different staged kernels: each
+    is timed."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    L.call("ctbb_set_autotune", 1)
+    try:
+        for i, fov in enumerate((50.0, 250.0)):
+            s = _scan(tmp_path / str(i), n=38, fov=fov)
+            _alone(torch, lib, s)
+            s.close()
+    finally:
+        L.call("ctbb_set_autotune", 0)
+    buf = C.create_string_buffer(1 << 16)
+    assert lib.ctbb_autotune_report(buf, len(buf)) > 0
+    entries = [e for e in buf.value.decode().splitlines() if e.startswith("38x38x32 ")]
+    assert len(entries) == 2, buf.value
