@@ -135,3 +135,32 @@ def test_windows_of_many_half_turns(box_check, tmp_path, z, rows, pitch, pixels,
     """A detector of few slices' height takes the staged form for small images only."""
     spec = scans.tiny(z, 0, n_rows_raw=rows, n_proj_turn=96, n_channels=128, nx=pixels, ny=pixels, n_slices=4, pitch=pitch)
     assert (_shape(box_check, spec, tmp_path)[0] > 0) == staged
+
+
+# what a scan's blocks run: channels, raw rows, z, phi, views, nx, ny, field of view, pitch, table -> columns / 32
+# of a tile, channels of its box
+TILES = {
+    "one_16x8_tile": ((64, 8, 0, 0, 96, 16, 8, 30.0, 1.0, "out"), (4, 56)),
+    "one_16x8_tile_wide_box": ((64, 8, 0, 0, 96, 16, 8, 60.0, 1.0, "in"), (4, 88)),
+    "half_a_tile": ((64, 8, 0, 0, 96, 8, 8, 30.0, 1.0, "out"), (4, 88)),
+    "past_a_tile": ((64, 8, 0, 0, 96, 17, 9, 40.0, 1.0, "out"), (4, 56)),
+    "8x8_tiles": ((256, 64, 0, 0, 100, 50, 47, 100.0, 1.1, "in"), (2, 88)),
+    "8x8_tiles_past_both": ((64, 8, 0, 0, 96, 9, 17, 60.0, 1.0, "out"), (2, 88)),
+    "8x8_tiles_2mm_pixels": ((128, 8, 1, 1, 96, 47, 50, 160.0, 1.0, "out"), (2, 88)),
+    "128_rows": ((64, 64, 1, 1, 192, 31, 33, 100.0, 0.8, "out"), (4, 56)),
+    "too_coarse": ((320, 8, 0, 0, 96, 47, 50, 100.0, 1.0, "out"), (0, 0)),
+    "rows_of_130": ((65, 16, 0, 0, 96, 20, 20, 30.0, 1.0, "out"), (0, 0)),
+}
+
+
+def tile_spec(name):
+    channels, rows, z, phi, views, nx, ny, fov, pitch, table = TILES[name][0]
+    spec = scans.tiny(z, phi, n_rows_raw=rows, n_proj_turn=views, n_channels=channels, nx=nx, ny=ny, n_slices=6,
+                      pitch=pitch, table_dir=table, seed=5)
+    spec.recon_fov = fov
+    return spec
+
+
+@pytest.mark.parametrize("name", TILES)
+def test_tile_of_a_block(box_check, tmp_path, name):
+    assert _shape(box_check, tile_spec(name), tmp_path) == TILES[name][1]
