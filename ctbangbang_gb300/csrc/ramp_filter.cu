@@ -838,11 +838,16 @@ int launch_ramp_filter(const RampFilterPlan &plan, float *d_lines, size_t n_line
         grid = (int)std::min<size_t>(n_pairs, (size_t)num_sms() * std::min(per_sm, 2));
         ramp_fft4096_kernel<2><<<grid, kFftThreads, smem, stream>>>(p, plan.d_tw16, plan.d_tw16 + 15 * 16);
     } else {
-        // a CTA to a pair while the GPU holds them all at once (three to an
-        // SM): 300 rows of 32 samples take 6 us so and 10 sharing CTAs, of 512
-        // 7 and 12; 1216 rows of 512 14 and 12
+        // Few pairs get a CTA each: up to the waves of three CTAs an SM at which
+        // that still is the faster way, by M = 256 (and below) .. 2048 -- the
+        // radix-2 and radix-8 passes of 512 and 2048 points are the longest for
+        // a pair's few threads.  us with a CTA to a pair / sharing, by rows:
+        // 96 samples, 300 6.2 / 8.2, 1500 10.3 / 8.2; 250, 900 8.0 / 14.4, 1500
+        // 10.9 / 14.4; 512, 900 8.2 / 12.3, 1500 14.4 / 14.4, 2400 20.5 / 14.4;
+        // 1024, 900 12.3 / 14.4, 2400 26.6 / 28.6, 4000 48.3 / 36.9.
+        constexpr int kOwnWaves[] = {1, 2, 1, 3};
         const int groups = kFftThreads / pair_threads(p.m);
-        const bool shared = groups > 1 && n_pairs > (size_t)num_sms() * 3;
+        const bool shared = groups > 1 && n_pairs > (size_t)num_sms() * 3 * kOwnWaves[std::max(p.log2m - 8, 0)];
         if (shared) {
             smem *= groups;
             per_sm = (int)std::min<size_t>(4, std::max<size_t>(1, (size_t)(220 * 1024) / smem));
