@@ -899,6 +899,34 @@ def measure_fp16(args, torch, lib, m, ref):
     return out
 
 
+# Parts of the line that only explain it: they go to stderr, so that the line on
+# stdout stays within a few KB (the tuner's report alone is 10).
+DETAIL = (("batch", "scans"), ("batch", "autotune"), ("serve", "scans"), ("serve", "per_scan_alone_ms"),
+          ("beside", "e2e", "breakdown_ms"), ("e2e", "breakdown_ms", "note"), ("fp16_storage", "roofline", "note"),
+          ("fp16_storage", "hu"), ("cpu_baseline", "sample"))
+
+
+def split_line(line):
+    """(line without its DETAIL parts and with 7-digit floats below the top
+    level, those parts by path)."""
+    def copied(v):
+        if isinstance(v, dict):
+            return {k: copied(x) for k, x in v.items()}
+        if isinstance(v, (list, tuple)):
+            return [copied(x) for x in v]
+        return float("%.7g" % v) if isinstance(v, float) and math.isfinite(v) else v
+
+    short = {k: v if isinstance(v, float) else copied(v) for k, v in line.items()}
+    detail = {}
+    for path in DETAIL:
+        at = short
+        for k in path[:-1]:
+            at = at.get(k) if isinstance(at, dict) else None
+        if isinstance(at, dict) and path[-1] in at:
+            detail[".".join(path)] = at.pop(path[-1])
+    return short, detail
+
+
 def run_ours(args):
     import torch
 
@@ -1057,6 +1085,8 @@ def run_ours(args):
         "gpu_launches": m["launches"] / args.steps,
         "clocks": m["clocks"],
     }
+    line, detail = split_line(line)
+    print(json.dumps(detail), file=sys.stderr, flush=True)
     print(json.dumps(line), flush=True)
     scans.free_plan(mr)
     if dist is not None:
