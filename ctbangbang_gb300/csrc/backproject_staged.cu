@@ -18,7 +18,7 @@
 // footprint is four gathers whose lanes fall on two rows of the same banks)
 // and close behind by issue (76 %).  Staged, the gathers take 1.2 wavefronts
 // each (rows 24 banks apart), the image sums cost no shared memory, classes
-// come from the visit list instead of votes, and the data pipe falls to 60 %;
+// come from the visit list instead of votes, and the data pipe falls to 66 %;
 // issue (77 %) and the wait for the slowest slice group of a step bound it.
 // Measured on a 32-slice block against the column form (ms): 512^2, 1472 x 128
 // rows, 3 half turns 12.10 -> 11.56; 512^2, 1472 x 64, 4 half turns 13.85 ->

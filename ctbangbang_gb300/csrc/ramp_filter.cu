@@ -10,10 +10,10 @@
 // GB300 design: FP32 FFT convolution in shared memory.  Two real rows are
 // packed into one complex row (x_a + i x_b); because the kernel is real the
 // real and imaginary parts of the inverse transform are the two filtered rows.
-// CTAs are persistent and loop over row pairs.  Row lengths 1025..1536 (every
+// CTAs are persistent and loop over row pairs.  Row lengths 1025..1535 (every
 // built-in scanner) take ramp_fft3072_kernel (16 x 16 x 12), see there; any M
 // of at least 2 N - 1 gives the same convolution.  For M = 4096 (row lengths
-// 1537..2048) ramp_fft4096_kernel runs 16 x 16 x 16
+// 1536..2048) ramp_fft4096_kernel runs 16 x 16 x 16
 // radix-16 passes: thread j owns butterfly j of every pass, the first forward
 // pass reads the rows from HBM (inputs >= M/2 are the zero padding), the last
 // forward pass, the spectrum multiply and the first inverse pass stay in
@@ -224,8 +224,8 @@ __device__ float2 *fft_smem(float2 *a, float2 *b, const float2 *tw, int m, int l
     return a;
 }
 
-// ---- 4096-point transforms (16 x 16 x 16): the size every row length in
-// 1025..2048 uses.  Thread j of 256 owns butterfly j of each pass; the three
+// ---- 4096-point transforms (16 x 16 x 16): the size row lengths 1536..2048
+// use.  Thread j of 256 owns butterfly j of each pass; the three
 // forward passes read inputs j + 256 r (r = 0..15), so the last forward pass
 // leaves X[j + 256 r] in thread j's registers -- exactly the inputs of the first
 // inverse pass.  Spectrum multiply and that pass run in registers; the first
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kFftThreads, MIN_BLOCKS)
     }
 }
 
-// ---- 3072-point transforms (16 x 16 x 12): row lengths 1025..1536.  A linear
+// ---- 3072-point transforms (16 x 16 x 12): row lengths 1025..1535.  A linear
 // convolution of N samples with 2 N - 1 taps needs M >= 2 N - 1 points, so 3072
 // serve these rows with three quarters of the 4096-point kernel's work.  The
 // same structure: inputs at M / 2 and beyond are the zero padding (first pass,
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kFftThreads, MIN_BLOCKS)
 // norm plain, 1.4e-7 as differences, for 4 % of the time).  Taken when F's white-noise gain is no larger than the taps'.
 //
 // Bound by the L1 data pipe
-// (70 %: shared-memory round trips and the twiddle tables) and the barriers
+// (77 %: shared-memory round trips and the twiddle tables) and the barriers
 // between passes, which four CTAs per SM (64 registers) overlap better than
 // three or two (40 001 rows of 1344: 270, 276 and 320 us; the 4096-point
 // kernel 313 us, at 9.3e-6).
