@@ -49,6 +49,7 @@
 #include <cstdlib>
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "ctbb_internal.h"
@@ -244,8 +245,12 @@ __device__ __forceinline__ void store4(float4 x, float s, __half *hi, __half *lo
 }
 
 // One warp per row: max |x|, its exponents, then x_hi, x_lo.  The row (at most
-// 1536 samples, a multiple of 64) is read once, into registers.
-template <bool VEC>
+// 1536 samples, a multiple of 64; at most 128 GROUPS) is read once, into
+// registers, and a short one into few: with room for 1536 samples a third of
+// the warps are resident and one load each is in flight (131 072 rows of 128,
+// with the filter: 120 us, 97 with two readings by scalar loads; 100 000 rows
+// as it is 75 us against 83, of 256 111 against 121, of 512 221 against 257).
+template <bool VEC, int GROUPS>
 __global__ void __launch_bounds__(256) ramp_tc_split_kernel(const float *__restrict__ x, size_t n_lines, int n,
                                                             float sum_abs_taps, __half *__restrict__ hi,
                                                             __half *__restrict__ lo, float *__restrict__ scale,
@@ -256,13 +261,13 @@ __global__ void __launch_bounds__(256) ramp_tc_split_kernel(const float *__restr
     const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
     for (size_t row = warp; row < n_lines; row += warps) {
         const float *xr = x + row * (size_t)n;
-        float4 v[kNPad / 128];
+        float4 v[GROUPS];
         float m = 0.0f;
 #pragma unroll
-        for (int k = 0; k < kNPad / 128; ++k)
+        for (int k = 0; k < GROUPS; ++k)
             if (4 * (lane + 32 * k) < n) v[k] = load4<VEC>(xr + 4 * (lane + 32 * k));
 #pragma unroll
-        for (int k = 0; k < kNPad / 128; ++k)
+        for (int k = 0; k < GROUPS; ++k)
             if (4 * (lane + 32 * k) < n) m = max4(m, v[k]);
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
         int e_in, e_out;
@@ -270,7 +275,7 @@ __global__ void __launch_bounds__(256) ramp_tc_split_kernel(const float *__restr
         if (lane == 0) write_scales(e_in, e_out, scale + row, mult + row);
         const float s = ldexpf(1.0f, -e_in);
 #pragma unroll
-        for (int k = 0; k < kNPad / 128; ++k) {
+        for (int k = 0; k < GROUPS; ++k) {
             const int i = 4 * (lane + 32 * k);
             if (i < n) store4(v[k], s, hi + row * (size_t)n + i, lo + row * (size_t)n + i);
         }
@@ -721,7 +726,14 @@ int launch_ramp_tc(const RampTcPlan &plan, const float *d_rows, size_t n_lines, 
                                                    d_scale, mult);
     } else {
         int blocks = (int)std::min<size_t>((n_lines + 7) / 8, (size_t)num_sms() * 16);
-        auto *split = vec ? ramp_tc_split_kernel<true> : ramp_tc_split_kernel<false>;
+        auto pick = [&](auto v) {
+            constexpr bool VEC = decltype(v)::value;
+            return n <= 128   ? ramp_tc_split_kernel<VEC, 1>
+                   : n <= 256 ? ramp_tc_split_kernel<VEC, 2>
+                   : n <= 512 ? ramp_tc_split_kernel<VEC, 4>
+                              : ramp_tc_split_kernel<VEC, kNPad / 128>;
+        };
+        auto *split = vec ? pick(std::true_type()) : pick(std::false_type());
         split<<<blocks, 256, 0, stream>>>(d_rows, n_lines, n, plan.sum_abs_taps, xh, xl, d_scale, mult);
     }
     count_launch();
