@@ -1423,9 +1423,10 @@ extern "C" int ctbb_batch_run(void)
             for (const auto &it : g_batch_items)
                 if (it.first == sh) group.push_back(it.second);
             CTBB_TRY(g_batch_params.ensure(backproject_batch_bytes(group.size())));
+            if (const size_t part = backproject_batch_partial_bytes(group, sh)) CTBB_TRY(c.bp_partial.ensure(part));
             StageScope scope(c, 3);
-            CTBB_TRY(launch_backproject_batch(group, sh, g_batch_params.ptr, g_batch_params.bytes, c.copy_error,
-                                              c.stream));
+            CTBB_TRY(launch_backproject_batch(group, sh, g_batch_params.ptr, g_batch_params.bytes, c.bp_partial.ptr,
+                                              c.bp_partial.bytes, c.copy_error, c.stream));
         }
         for (size_t s = 0; s < g_batch.size(); ++s)
             CTBB_TRY(do_finalize(c, *g_batch[s].mr, g_slots[s].image.as<float>(), g_batch[s].d_final,

@@ -718,6 +718,21 @@ __global__ void backproject_combine_kernel(const float *__restrict__ partial, fl
     }
 }
 
+// The same for the blocks of a batch (grid y).
+__global__ void backproject_combine_batch_kernel(const BpParams *__restrict__ params, int chunks)
+{
+    const BpParams &p = params[blockIdx.y];
+    const float *partial = p.partial;
+    float *out = p.out;
+    const float scale = p.out_scale;
+    const size_t n = (size_t)p.n_slices * p.nx * p.ny;
+    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
+        float s = partial[v];
+        for (int c = 1; c < chunks; ++c) s += partial[(size_t)c * n + v];
+        out[v] = s * scale;
+    }
+}
+
 // Dynamic shared memory of the column form: a geometry entry (24 bytes) per
 // thread and half turn of the window (at most nht).
 __host__ __device__ constexpr size_t column_geo_bytes(int nht, int threads)
@@ -1263,22 +1278,44 @@ int staged_block_chunks(const BpParams &p, const StagedShape &s, int limit)
     return chunks <= p.n_half ? chunks : 1;
 }
 
-// The blocks of a batch that take the staged form: those of one staged shape
-// and one number of angle chunks together, one launch per chunk.  A block has
-// the chunks it has alone, so that its image is the same sum.
-int launch_staged_batch(const std::vector<BpParams> &blocks, int limit, void *d_buf, size_t buf_bytes,
-                        CopyError &errors, cudaStream_t stream)
+// The blocks of a batch that take the staged form, by staged shape and number of
+// angle chunks.
+using StagedKind = std::pair<StagedShape, int>;
+int staged_kinds(const std::vector<BpParams> &blocks, int limit, std::vector<StagedKind> *kind_of,
+                 std::vector<StagedKind> *kinds)
 {
-    using Kind = std::pair<StagedShape, int>;
-    std::vector<Kind> kind_of(blocks.size()), kinds;
+    kind_of->resize(blocks.size());
     for (size_t b = 0; b < blocks.size(); ++b) {
-        if (!staged_shape(blocks[b], &kind_of[b].first)) {
+        StagedKind &k = (*kind_of)[b];
+        if (!staged_shape(blocks[b], &k.first)) {
             set_error("backproject batch: a block does not fit the staged form");
             return CTBB_ERR_ARGUMENT;
         }
-        kind_of[b].second = staged_block_chunks(blocks[b], kind_of[b].first, limit);
-        if (std::find(kinds.begin(), kinds.end(), kind_of[b]) == kinds.end()) kinds.push_back(kind_of[b]);
+        k.second = staged_block_chunks(blocks[b], k.first, limit);
+        if (std::find(kinds->begin(), kinds->end(), k) == kinds->end()) kinds->push_back(k);
     }
+    return CTBB_OK;
+}
+
+// Whether the blocks of a kind run all their angle chunks in one launch, which
+// writes partial sums, instead of one launch per chunk: below two CTAs for every
+// place of 152 SMs, where the launches in series leave SMs idle (at most 160 MB
+// of sums).  Batches, one launch per chunk / at once: two scans of 16^2, 40 half
+// turns, 1378 / 273 us (667 in the slice-chunk form, one launch); two of 100^2,
+// 16 rows 9.5 / 7.0 ms (10.6 in the column form).
+constexpr unsigned kChunksAtOnce = 608;
+
+size_t block_partial_floats(const BpParams &p, int n_ac) { return (size_t)n_ac * p.n_slices * p.nx * p.ny; }
+
+// The blocks of a batch that take the staged form: those of one kind together,
+// in one launch per chunk, or one in all.  A block has the chunks it has alone,
+// so that its image is the same sum.
+int launch_staged_batch(const std::vector<BpParams> &blocks, int limit, void *d_buf, size_t buf_bytes, void *scratch,
+                        size_t scratch_bytes, CopyError &errors, cudaStream_t stream)
+{
+    using Kind = StagedKind;
+    std::vector<Kind> kind_of, kinds;
+    CTBB_TRY(staged_kinds(blocks, limit, &kind_of, &kinds));
     if (backproject_batch_bytes(blocks.size()) > buf_bytes) {
         set_error("backproject batch: parameter buffer too small");
         return CTBB_ERR_ARGUMENT;
@@ -1302,6 +1339,13 @@ int launch_staged_batch(const std::vector<BpParams> &blocks, int limit, void *d_
             }
             start.push_back((unsigned)next);
         }
+        bool at_once = n_ac > 1 && start.back() < kChunksAtOnce && scratch;
+        size_t floats = 0;
+        for (BpParams &p : group) {
+            p.partial = static_cast<float *>(scratch) + floats;
+            floats += block_partial_floats(p, n_ac);
+        }
+        at_once = at_once && floats * sizeof(float) <= scratch_bytes;
         char *d_maps = static_cast<char *>(d_buf);
         BpParams *d_params = reinterpret_cast<BpParams *>(d_maps + maps.size());
         unsigned *d_start = reinterpret_cast<unsigned *>(d_params + group.size());
@@ -1310,20 +1354,48 @@ int launch_staged_batch(const std::vector<BpParams> &blocks, int limit, void *d_
                                       stream));
         CTBB_CUDA_TRY(cudaMemcpyAsync(d_start, start.data(), start.size() * sizeof(unsigned), cudaMemcpyHostToDevice,
                                       stream));
-        for (int ac = 0; ac < n_ac; ++ac)
+        for (int ac = at_once ? -1 : 0; ac < (at_once ? 0 : n_ac); ++ac)
             CTBB_TRY(launch_backproject_staged_batch(d_params, d_start, d_maps, start.back(), (int)group.size(), ac,
                                                      n_ac, shape, errors, stream));
+        if (at_once) {
+            size_t most = 0;
+            for (const BpParams &p : group) most = std::max(most, block_partial_floats(p, 1));
+            const dim3 grid((unsigned)std::min<size_t>((most + 255) / 256, 152 * 16), (unsigned)group.size());
+            backproject_combine_batch_kernel<<<grid, 256, 0, stream>>>(d_params, n_ac);
+            count_launch();
+            CTBB_CUDA_TRY(cudaGetLastError());
+        }
     }
     return CTBB_OK;
 }
 
 }  // namespace
 
+size_t backproject_batch_partial_bytes(const std::vector<BpParams> &blocks, const BpShape &shape)
+{
+    std::vector<StagedKind> kind_of, kinds;
+    if (!shape.staged || staged_kinds(blocks, shape.staged, &kind_of, &kinds) != CTBB_OK) return 0;
+    size_t most = 0;
+    for (const StagedKind &kind : kinds) {
+        if (kind.second <= 1) continue;
+        unsigned long long tiles = 0;
+        size_t floats = 0;
+        for (size_t b = 0; b < blocks.size(); ++b)
+            if (kind_of[b] == kind) {
+                tiles += staged_tiles(blocks[b], kind.first);
+                floats += block_partial_floats(blocks[b], kind.second);
+            }
+        if (tiles < kChunksAtOnce) most = std::max(most, floats * sizeof(float));
+    }
+    return most;
+}
+
 int launch_backproject_batch(const std::vector<BpParams> &blocks, const BpShape &shape, void *d_buf, size_t buf_bytes,
-                             CopyError &errors, cudaStream_t stream)
+                             void *scratch, size_t scratch_bytes, CopyError &errors, cudaStream_t stream)
 {
     if (blocks.empty()) return CTBB_OK;
-    if (shape.staged) return launch_staged_batch(blocks, shape.staged, d_buf, buf_bytes, errors, stream);
+    if (shape.staged)
+        return launch_staged_batch(blocks, shape.staged, d_buf, buf_bytes, scratch, scratch_bytes, errors, stream);
     const bool quad = blocks[0].vscale != nullptr;
     for (const BpParams &p : blocks)
         if ((p.vscale != nullptr) != quad || p.nos != blocks[0].nos) {

@@ -97,7 +97,8 @@ struct StagedShape {
 // more than 32 slices, voxels near the source's circle).
 bool staged_shape(const BpParams &p, StagedShape *out);
 int launch_backproject_staged(const BpParams &p, const StagedShape &s, CopyError &errors, cudaStream_t stream);
-// Angle chunk ac of n_ac of n blocks of one staged shape, total CTA tiles.
+// Angle chunk ac of n_ac of n blocks of one staged shape, total CTA tiles; ac <
+// 0: all chunks at once, as partial sums in each block's `partial`.
 // d_maps: the blocks' TMA descriptors (staged_map, staged_map_bytes() each, 64-byte aligned).
 int launch_backproject_staged_batch(const BpParams *d_params, const unsigned *d_start, const void *d_maps,
                                     unsigned total, int n, int ac, int n_ac, const StagedShape &s,
@@ -136,14 +137,17 @@ int launch_backproject_params(const BpParams &p, const BpShape &shape, CopyError
                               void *scratch = nullptr, size_t scratch_bytes = 0);
 // Bytes of partial image sums a launch of this shape needs (0: none).
 size_t backproject_partial_bytes(const BpParams &p, const BpShape &shape);
-// Device bytes launch_backproject_batch needs for n blocks' parameters.
+// Device bytes launch_backproject_batch needs for n blocks' parameters, and for
+// the partial image sums of the blocks that run their angle chunks at once.
 size_t backproject_batch_bytes(size_t n_blocks);
+size_t backproject_batch_partial_bytes(const std::vector<BpParams> &blocks, const BpShape &shape);
 // All blocks (of any scans; one row storage and row length) in one launch of
 // the given shape -- the column form one launch per angle chunk, each adding
 // to the blocks' images in chunk order; d_buf holds
-// backproject_batch_bytes(blocks.size()).
+// backproject_batch_bytes(blocks.size()), scratch the partial sums.
 int launch_backproject_batch(const std::vector<BpParams> &blocks, const BpShape &shape, void *d_buf,
-                             size_t buf_bytes, CopyError &errors, cudaStream_t stream);
+                             size_t buf_bytes, void *scratch, size_t scratch_bytes, CopyError &errors,
+                             cudaStream_t stream);
 int launch_backproject(const struct recon_metadata &mr, const BackprojectTables &t,
                        const float4 *d_views, const float *d_theta, const float *d_zpos, const float *d_rebin,
                        float *d_block, int zpt, CopyError &errors, cudaStream_t stream,

@@ -479,7 +479,8 @@ __global__ void __launch_bounds__(128 * CW, 8 / CW) backproject_staged_kernel(Bp
 }
 
 // The blocks of a batch in one launch per angle chunk (see
-// backproject_column_batch_kernel).
+// backproject_column_batch_kernel), or, ac < 0, with grid y over the chunks,
+// which write partial sums.
 template <int CW, int PITCH>
 __global__ void __launch_bounds__(128 * CW, 8 / CW)
     backproject_staged_batch_kernel(const BpParams *__restrict__ params, const unsigned *__restrict__ tile_start,
@@ -509,9 +510,12 @@ __global__ void __launch_bounds__(128 * CW, 8 / CW)
                  : "memory");
     const unsigned local = tile - __ldg(tile_start + b);
     const unsigned gx = (unsigned)((sp.nx + tile_x(CW) - 1) / tile_x(CW));
-    const int mode = n_ac == 1 ? kOutScaled : ac == 0 ? kOutFirst : ac == n_ac - 1 ? kOutLast : kOutMiddle;
-    backproject_staged_tile<CW, PITCH>(sp, (int)(local % gx), (int)(local / gx), ac, n_ac, mode, lay,
-                                             maps + b, error);
+    const int mode = ac < 0      ? kOutPartial
+                     : n_ac == 1 ? kOutScaled
+                     : ac == 0   ? kOutFirst
+                                 : (ac == n_ac - 1 ? kOutLast : kOutMiddle);
+    backproject_staged_tile<CW, PITCH>(sp, (int)(local % gx), (int)(local / gx), ac < 0 ? (int)blockIdx.y : ac, n_ac,
+                                             mode, lay, maps + b, error);
 }
 
 // Calls f(CW, PITCH) with a shape's compile-time instance.
@@ -662,8 +666,8 @@ int launch_backproject_staged_batch(const BpParams *d_params, const unsigned *d_
         const StagedLayout lay = staged_layout(CW, s.half_bytes);
         CTBB_TRY(raise_smem_limit(reinterpret_cast<const void *>(backproject_staged_batch_kernel<CW, PITCH>)));
         backproject_staged_batch_kernel<CW, PITCH>
-            <<<total, 128 * CW, lay.total, stream>>>(d_params, d_start, static_cast<const CUtensorMap *>(d_maps), n, ac,
-                                                     n_ac, lay, err);
+            <<<dim3(total, ac < 0 ? n_ac : 1), 128 * CW, lay.total, stream>>>(
+                d_params, d_start, static_cast<const CUtensorMap *>(d_maps), n, ac, n_ac, lay, err);
         count_launch();
         CTBB_CUDA_TRY(cudaGetLastError());
         return CTBB_OK;
