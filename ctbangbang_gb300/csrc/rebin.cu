@@ -487,9 +487,9 @@ __global__ void rebin_two_stage_kernel(RebinParams p)
 // consecutive channels do not collide.  Same taps, same arithmetic, same bits.
 // Small tiles: t_alpha's span over a tile adds frames to every box, so 128
 // channels (96 KB of boxes, 2 CTAs per SM) moved 3.2 GB from L2 and took 592
-// us on a config-2 window where 64 (37 KB, 6 CTAs) move 2.55 GB and take 415;
-// 32 views to a box 550, 256 threads 454; gathering 611.  What bounds it now
-// is the L2 traffic of the boxes (6.1 TB/s) beside 4.9 TB/s of HBM.
+// us on a config-2 window where 64 (37 KB, 6 CTAs) move 2.55 GB and took 415
+// (390 now); 32 views to a box 550, 256 threads 454; gathering 611.  What bounds
+// it now is the L2 traffic of the boxes (6.6 TB/s) beside 5.2 TB/s of HBM.
 constexpr int kNarrowBox = 40, kWideBox = 48;  // channels of a box: a tile's, wider with a z flying focal spot
 
 struct StagedRebin {
